@@ -91,3 +91,31 @@ def test_coordination_needs_a_single_scene(engine_lib):
         b.coordination()
     assert ex.value.code == 1
     b.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 1500])
+@pytest.mark.parametrize("far", [0.0, 1.0, 1e4])
+def test_device_coordination_where_each_of_its_tests_decides(n, far, engine_lib, port_lib):
+    """Polydisperse touching spheres (exact ties among them), some pulled apart or together by one
+    part in 1e6 to 1e12, with one sphere `far` metres away: the wider the scene, the fewer pairs the
+    FP32 and the double-float test may decide.  Every count equals the oracle's."""
+    from oracle import PortWorld
+    rng = np.random.default_rng(n)
+    sc = scenes.cluster(n=n, seed=n, polydisperse=True, walls="none")
+    r = np.array([sc.models[m].attrs[0] for m in sc.model_index])
+    x = np.zeros((n, 3))
+    for i in range(1, n):                      # three touching chains side by side
+        row, prev = i % 3, i - 3
+        d = (r[i] + r[prev]) * (1.0 + rng.choice([0.0, 1e-12, -1e-12, 1e-9, -1e-9, 1e-6, -1e-6])) if prev >= 0 else 0.0
+        x[i] = [(x[prev, 0] + d) if prev >= 0 else 0.0, 1.9e-3 * row, 1e-4 * row]
+    if far and n > 2:
+        x[n // 2, 2] += far
+    sc.position[:] = x
+    e = engine_lib.GpuEngine(sc)
+    box = (x[:, 0].min(), x[:, 0].mean() + 1e-4, -1.0, 1.0, -1.0, 1.0)
+    below, touching, avg = e.coordination(box)
+    pb, pt, pavg = PortWorld(sc).coordination(box)
+    np.testing.assert_array_equal(below, pb)
+    np.testing.assert_array_equal(touching, pt)
+    assert avg == pavg or (np.isnan(avg) and np.isnan(pavg))
+    e.close()

@@ -117,6 +117,7 @@ private:
     uint32_t* d_global_ = nullptr;
     // device: broad-phase scratch
     Scratch scratch_;
+    Scratch cn_;                         // the coordination numbers' workspace
     double* d_safe_ = nullptr;
     unsigned long long* d_red_ = nullptr;
     uint64_t *d_key_ = nullptr, *d_key_alt_ = nullptr, *d_cell_key_ = nullptr;

@@ -20,6 +20,7 @@ struct DeviceObjects {
     const double4_32a* pos = nullptr;
     cudaStream_t stream = nullptr;
     Scratch* scratch = nullptr;
+    Scratch* work = nullptr;             // the coordination numbers' workspace, kept by the engine
     const HScene* scene = nullptr;       // the models and object order of the scene
     uint64_t* launches = nullptr;        // the engine's kernel launch counter
 };

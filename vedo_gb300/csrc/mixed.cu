@@ -42,6 +42,7 @@
 #include <cuda_runtime.h>
 
 #include "dem_common.cuh"
+#include "dfloat.cuh"
 #include "engine_base.h"
 #include "observables.cuh"
 #include "prefilter.cuh"
@@ -195,29 +196,6 @@ __device__ __forceinline__ f3 fcross(f3 a, f3 b) {
 }
 __device__ __forceinline__ f3 f4to3(float4 v) { return fm(v.x, v.y, v.z); }
 
-// Double-float (hi + lo, ~48 bits) arithmetic from error-free FP32 transforms (Knuth's two-sum,
-// the FMA two-product).  Both spheres' positions are split into hi/lo FP32 pairs (split32 below),
-// then the relative displacement, |d|^2 and the overlap numerator R^2 - |d|^2 need no FP64 work.
-// The splits are either stored once per step (xs arrays) or formed when a pair needs them: the
-// same function on the same FP64 positions, so the two ways give identical bits.
-struct dfl { float hi, lo; };
-__device__ __forceinline__ dfl two_sum(float a, float b) {
-    const float s = a + b, bb = s - a;
-    return dfl{s, (a - (s - bb)) + (b - bb)};
-}
-__device__ __forceinline__ dfl df_add(dfl a, dfl b) {
-    const dfl s = two_sum(a.hi, b.hi);
-    return two_sum(s.hi, s.lo + (a.lo + b.lo));
-}
-// (hm + lm) - (hs + ls)
-__device__ __forceinline__ dfl df_diff(float hm, float lm, float hs, float ls) {
-    const dfl d = two_sum(hm, -hs);
-    return two_sum(d.hi, d.lo + (lm - ls));
-}
-__device__ __forceinline__ dfl df_sq(dfl a) {
-    const float p = a.hi * a.hi;
-    return two_sum(p, fmaf(a.hi, a.hi, -p) + 2.0f * a.hi * a.lo);
-}
 // The nearest periodic image of a double-float difference on an axis of range L (FP32, 0 = off;
 // Lhi + Llo = the FP64 range): one range off when the difference reaches half of it, as
 // Boundary::DifferenceBoundaryConditions does (pairs that can touch are far from that limit).
@@ -227,38 +205,6 @@ __device__ __forceinline__ dfl df_image(dfl d, float L, float Lhi, float Llo) {
     if (v >= 0.5f * L) return df_add(d, dfl{-Lhi, -Llo});
     if (v < -0.5f * L) return df_add(d, dfl{Lhi, Llo});
     return d;
-}
-
-// x = hi + lo with hi = x rounded to FP32 (nearest, ties to even) and lo = (x - hi) rounded to
-// FP32, from the bits of x with integer operations (GB300's FP64 pipe is its scarcest): for
-// 2^-70 <= |x| < 2^101; zero, tiny and huge values take the FP64 conversions.
-// The FP64 conversions of the rare exponents, out of line: GB300 issues FP64 conversions on its
-// FP64 pipe (2 lanes per cycle per SM), and a short branch kept inline is predicated rather than
-// jumped over, so its FP64 instructions would be issued on every call.
-__device__ __noinline__ void split32_wide(double x, float& hi, float& lo) {
-    hi = (float)x;
-    lo = (float)(x - (double)hi);
-}
-__device__ __forceinline__ void split32(double x, float& hi, float& lo) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    const int e = (int)((u >> 52) & 0x7ff) - 1023;           // unbiased exponent
-    if (e < -70 || e > 100) {                                  // 2^(e-52) below stays a normal FP32
-        split32_wide(x, hi, lo);
-        return;
-    }
-    const unsigned long long mant = u & 0xfffffffffffffull;   // 52 bits
-    const unsigned sign = (unsigned)(u >> 63) << 31;
-    const unsigned m23 = (unsigned)(mant >> 29);
-    const unsigned rem = (unsigned)(mant & 0x1fffffffu);      // 29 bits below FP32's mantissa
-    const bool up = rem > 0x10000000u || (rem == 0x10000000u && (m23 & 1u));
-    // exponent and mantissa as one integer: a carry out of the mantissa bumps the exponent
-    const unsigned body = (((unsigned)(e + 127)) << 23) + m23 + (up ? 1u : 0u);
-    hi = __uint_as_float(sign | body);
-    // x - hi = (rem or rem - 2^29) units of 2^(e - 52), exactly; its FP32 rounding
-    const int r = up ? (int)rem - (int)0x20000000 : (int)rem;
-    const float unit = __uint_as_float((unsigned)(e - 52 + 127) << 23);   // 2^(e-52)
-    const float lr = __int2float_rn(r) * unit;
-    lo = r == 0 ? 0.0f : (sign ? -lr : lr);                     // x - hi = +0 when exact
 }
 
 // Exact FP32 <-> FP64 conversions from the bits, with integer operations: the same values as the
@@ -2850,6 +2796,7 @@ private:
     NList nl_[2];
     int nlc_ = 0;                   // current neighbour list
     Scratch scratch_;
+    Scratch cn_;                    // the coordination numbers' workspace
     uint64_t *d_key_ = nullptr, *d_key_alt_ = nullptr;
     uint32_t *d_sid_ = nullptr, *d_sid_alt_ = nullptr, *d_cnt_ = nullptr;
     uint32_t *d_gs_ = nullptr, *d_ge_ = nullptr;
@@ -4415,7 +4362,7 @@ int MixedEngine::caller_view() {
 DeviceObjects MixedEngine::objects() {
     DeviceObjects d;
     d.n = n_; d.model_of = d_model_e_; d.models = d_models_; d.pos = d_xe_;
-    d.stream = stream_; d.scratch = &scratch_; d.launches = &launches_;
+    d.stream = stream_; d.scratch = &scratch_; d.work = &cn_; d.launches = &launches_;
     d.scene = sc_.size() == 1 ? host_[0].get() : nullptr;
     return d;
 }
