@@ -1649,19 +1649,19 @@ int Engine::get_interactions(const vedo_contact_view& v) {
 }
 
 int Engine::get_observables(double out[13]) {
-    const unsigned nb = std::max(1u, blocks_for(n_));
+    const unsigned nb = obs::obs_blocks(n_);
     double* part = d_obs_;
     double* res = d_obs_ + (size_t)nb * 16 + 16;
     const d3 g = mk(g_[0], g_[1], g_[2]);
     obs::k_obs_a<<<nb, TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_pos_, d_vel_, d_av_, g, part);
-    obs::k_obs_reduce<<<1, 32, 0, stream_>>>(nb, 16, part, res, 12);
+    obs::k_obs_reduce<<<16, TPB, 0, stream_>>>(nb, 16, part, res, 12);
     if (cur_.np)
         k_detect_active<<<blocks_for(cur_.np), TPB, 0, stream_>>>(cur_.np, cur_.sm, cur_.param, d_params_, d_geom_,
                                                                   d_hole_, d_reach_, d_pos_, d_ox_, d_oz_, d_pos32_,
                                                                   d_wall32_, cur_.flags, tab_.pbc);
-    obs::k_obs_b<<<nb, TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_pos_, d_vel_, d_av_, res, 0, cur_.flags, cur_.np,
-                                     part);
-    obs::k_obs_reduce<<<1, 32, 0, stream_>>>(nb, 6, part, res + 16, 6);
+    obs::k_obs_b<<<nb, TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_pos_, d_vel_, d_av_, res, cur_.flags, cur_.np,
+                                          part);
+    obs::k_obs_reduce<<<6, TPB, 0, stream_>>>(nb, 6, part, res + 16, 6);
     double r[22];
     CK(cudaMemcpyAsync(r, res, sizeof(r), cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
