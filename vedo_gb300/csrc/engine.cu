@@ -10,7 +10,7 @@
 //   k_obj   - one thread per local object: the pair impulses in candidate-list order
 //             (the reference's IactContainer order), the field impulse, the external
 //             force and DiscreteObject::Response.  Scope-global objects (walls) are
-//             summed by one warp each in k_obj_global (ordered, warp-cooperative loads).
+//             summed by one block each (ordered additions, cooperative loads).
 // Every UpIact steps the candidate list is rebuilt with NBSConsultant's rule
 // (NBSConsultant.cpp:85-374): cell keys, a stable radix sort, cell ranges, then a count
 // and a fill pass over (object, neighbour slot) tasks laid out in the reference's
@@ -331,104 +331,128 @@ __device__ __forceinline__ void finish_object(uint32_t i, const ModelDev& m, d3 
     }
 }
 
-__global__ void __launch_bounds__(TPB) k_obj(uint32_t n, const uint32_t* __restrict__ model_of,
-                                             const ModelDev* __restrict__ models, double4_32a* __restrict__ pos,
-                                             double4_32a* __restrict__ vel, double4_32a* __restrict__ av,
-                                             double4_32a* __restrict__ ox, double4_32a* __restrict__ oz,
-                                             double4_32a* __restrict__ imp, double4_32a* __restrict__ aimp,
-                                             const uint32_t* __restrict__ csr_ptr, const uint32_t* __restrict__ csr_ent,
-                                             const uint8_t* __restrict__ flags, const double* __restrict__ out,
-                                             double dt, d3 fimp, int write_imp, d3 origin, float4* __restrict__ pos32,
-                                             float4* __restrict__ wall32, const double* __restrict__ ext_imp,
-                                             const double* __restrict__ ext_aimp, Periodic pb,
-                                             uint8_t* __restrict__ touched, uint32_t* __restrict__ nwork) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) *nwork = 0u;                                   // the pair worklist, empty for the next step
-    if (i >= n) return;
-    const ModelDev& m = models[model_of[i]];
+struct ObjArgs {
+    uint32_t n;
+    const uint32_t* model_of;
+    const ModelDev* models;
+    double4_32a *pos, *vel, *av, *ox, *oz, *imp, *aimp;
+    const uint32_t *csr_ptr, *csr_ent;
+    const uint8_t* flags;
+    const double* out;
+    double dt;
+    d3 fimp;
+    int write_imp;
+    d3 origin;
+    float4 *pos32, *wall32;
+    const double *ext_imp, *ext_aimp;
+    Periodic pb;
+    uint8_t* touched;
+    uint32_t* nwork;
+    uint32_t nglob;
+    const uint32_t* glob;
+};
+
+// One block per scope-global object, when its sum is wanted (its impulse is written, or it responds):
+// the entries that applied an impulse, added in entry order, which keeps the reference's summation
+// order.  Only the additions are serial: seven warps load and compact the next 224 entries into
+// shared memory while the first warp adds the present ones, one component a lane, so that an entry
+// costs one dependent FP64 addition.  (One warp that did both, with every lane adding all six
+// components from shuffles, took 0.91 ms on the walls of 300,000 packed spheres.)
+constexpr int GSUM_TILE = TPB - 32;
+__device__ __forceinline__ void global_object(const ObjArgs& a, uint32_t i) {
+    __shared__ double buf[2][GSUM_TILE][6];
+    __shared__ uint32_t cnt[2], warp_cnt[GSUM_TILE / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0 && a.touched[i]) a.touched[i] = 0;
+    const ModelDev& m = a.models[a.model_of[i]];
+    double sum = 0.0;                          // component `lane` of (J, JA) in the first warp
+    if (a.write_imp || m.behavior == BEH_MOBILE || m.behavior == BEH_CONSTRAINED || a.ext_imp) {
+        const uint32_t e0 = a.csr_ptr[i], e1 = a.csr_ptr[i + 1];
+        const uint32_t tiles = (e1 - e0 + GSUM_TILE - 1) / GSUM_TILE;
+        for (uint32_t t = 0; t <= tiles; ++t) {            // load tile t, add tile t - 1
+            if (warp > 0 && t < tiles) {
+                const uint32_t e = e0 + t * GSUM_TILE + (threadIdx.x - 32);
+                uint32_t ent = 0;
+                uint8_t f = 0;
+                if (e < e1) {
+                    ent = a.csr_ent[e];
+                    f = a.flags[ent >> 1];
+                }
+                const bool app = f & PF_APPLIED;
+                const unsigned am = __ballot_sync(0xffffffffu, app);
+                if (lane == 0) warp_cnt[warp - 1] = (uint32_t)__popc(am);
+                asm volatile("bar.sync 1, 224;" ::: "memory");       // the loading warps
+                uint32_t at = (uint32_t)__popc(am & ((1u << lane) - 1u)), total = 0;
+                for (int w = 0; w < GSUM_TILE / 32; ++w) {
+                    if (w < warp - 1) at += warp_cnt[w];
+                    total += warp_cnt[w];
+                }
+                if (threadIdx.x == 32) cnt[t & 1] = total;
+                if (app) {
+                    const double* o = a.out + 9 * (size_t)(ent >> 1);
+                    double* d = buf[t & 1][at];
+                    const bool master = ent & 1;           // B->AddImpact(-1.0 * ImpactA, tB), else A->AddImpact(ImpactA, tA)
+                    for (int k = 0; k < 3; ++k) d[k] = master ? -o[k] : o[k];
+                    // (an impulse without a torque adds +0, which leaves a sum that started at +0 as it is)
+                    for (int k = 0; k < 3; ++k) d[3 + k] = f & PF_ANGULAR ? o[(master ? 6 : 3) + k] : 0.0;
+                }
+            }
+            if (warp == 0 && t > 0 && lane < 6) {
+                const uint32_t c = cnt[(t - 1) & 1];
+#pragma unroll 8
+                for (uint32_t k = 0; k < c; ++k) sum = sum + buf[(t - 1) & 1][k][lane];
+            }
+            __syncthreads();
+        }
+    }
+    if (warp != 0) return;
+    d3 J, JA;
+    J.x = __shfl_sync(0xffffffffu, sum, 0);
+    J.y = __shfl_sync(0xffffffffu, sum, 1);
+    J.z = __shfl_sync(0xffffffffu, sum, 2);
+    JA.x = __shfl_sync(0xffffffffu, sum, 3);
+    JA.y = __shfl_sync(0xffffffffu, sum, 4);
+    JA.z = __shfl_sync(0xffffffffu, sum, 5);
+    if (lane == 0)
+        finish_object(i, m, J, JA, a.dt, a.fimp, a.pos, a.vel, a.av, a.ox, a.oz, a.imp, a.aimp, a.write_imp, a.origin,
+                      a.pos32, a.wall32, a.ext_imp, a.ext_aimp, a.pb);
+}
+
+// The first nglob blocks take the scope-global objects (no object reads another's state here, so the
+// two run side by side in one launch), the others the local objects, one per thread.
+__global__ void __launch_bounds__(TPB) k_obj(ObjArgs a) {
+    if (blockIdx.x < a.nglob) {
+        global_object(a, a.glob[blockIdx.x]);
+        return;
+    }
+    const uint32_t i = (blockIdx.x - a.nglob) * blockDim.x + threadIdx.x;
+    if (i == 0) *a.nwork = 0u;                                 // the pair worklist, empty for the next step
+    if (i >= a.n) return;
+    const ModelDev& m = a.models[a.model_of[i]];
     if (m.scope == SCOPE_GLOBAL) return;
     d3 J = mk(0.0, 0.0, 0.0), JA = mk(0.0, 0.0, 0.0);
     // an object no pair applied an impulse to keeps zero sums: its ordered walk adds nothing
-    if (touched[i]) {
-        touched[i] = 0;
-        const uint32_t e0 = csr_ptr[i], e1 = csr_ptr[i + 1];
+    if (a.touched[i]) {
+        a.touched[i] = 0;
+        const uint32_t e0 = a.csr_ptr[i], e1 = a.csr_ptr[i + 1];
         // the entries that applied an impulse are marked first (integer work), then summed in entry
         // order: a warp issues each FP64 add once per marked entry of its busiest object, not once
         // per candidate entry (most candidates of an object apply nothing)
         const uint32_t c1 = min(e1, e0 + 64u);
         unsigned long long mark = 0ull;
         for (uint32_t e = e0; e < c1; ++e)
-            if (flags[csr_ent[e] >> 1] & PF_APPLIED) mark |= 1ull << (e - e0);
+            if (a.flags[a.csr_ent[e] >> 1] & PF_APPLIED) mark |= 1ull << (e - e0);
         for (; mark; mark &= mark - 1) {
-            const uint32_t ent = csr_ent[e0 + (uint32_t)(__ffsll(mark) - 1)];
-            add_entry(ent, flags[ent >> 1], out, J, JA);
+            const uint32_t ent = a.csr_ent[e0 + (uint32_t)(__ffsll(mark) - 1)];
+            add_entry(ent, a.flags[ent >> 1], a.out, J, JA);
         }
         for (uint32_t e = c1; e < e1; ++e) {                   // long lists: the entries after 64
-            const uint32_t ent = csr_ent[e];
-            add_entry(ent, flags[ent >> 1], out, J, JA);
+            const uint32_t ent = a.csr_ent[e];
+            add_entry(ent, a.flags[ent >> 1], a.out, J, JA);
         }
     }
-    finish_object(i, m, J, JA, dt, fimp, pos, vel, av, ox, oz, imp, aimp, write_imp, origin, pos32, wall32, ext_imp,
-                  ext_aimp, pb);
-}
-
-// One warp per scope-global object: lanes load 32 entries at a time, then every lane adds
-// them in order (shuffle broadcast), which keeps the reference's summation order.
-__global__ void k_obj_global(uint32_t nglob, const uint32_t* __restrict__ glob, const uint32_t* __restrict__ model_of,
-                             const ModelDev* __restrict__ models, double4_32a* __restrict__ pos,
-                             double4_32a* __restrict__ vel, double4_32a* __restrict__ av, double4_32a* __restrict__ ox,
-                             double4_32a* __restrict__ oz, double4_32a* __restrict__ imp, double4_32a* __restrict__ aimp,
-                             const uint32_t* __restrict__ csr_ptr, const uint32_t* __restrict__ csr_ent,
-                             const uint8_t* __restrict__ flags, const double* __restrict__ out, double dt, d3 fimp,
-                             int write_imp, d3 origin, float4* __restrict__ pos32, float4* __restrict__ wall32,
-                             const double* __restrict__ ext_imp, const double* __restrict__ ext_aimp, Periodic pb,
-                             uint8_t* __restrict__ touched) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= nglob) return;
-    const uint32_t i = glob[w];
-    if (lane == 0 && touched[i]) touched[i] = 0;
-    const ModelDev& m = models[model_of[i]];
-    d3 J = mk(0.0, 0.0, 0.0), JA = mk(0.0, 0.0, 0.0);
-    const bool need_sum = write_imp || m.behavior == BEH_MOBILE || m.behavior == BEH_CONSTRAINED || ext_imp;
-    if (need_sum) {
-        const uint32_t e0 = csr_ptr[i], e1 = csr_ptr[i + 1];
-        for (uint32_t base = e0; base < e1; base += 32) {
-            const uint32_t e = base + lane;
-            double jx = 0, jy = 0, jz = 0, ax = 0, ay = 0, az = 0;
-            int app = 0;
-            if (e < e1) {
-                const uint32_t ent = csr_ent[e];
-                const uint8_t f = flags[ent >> 1];
-                if (f & PF_APPLIED) {
-                    const double* o = out + 9 * (size_t)(ent >> 1);
-                    app = 1;
-                    if (ent & 1) {
-                        jx = -o[0]; jy = -o[1]; jz = -o[2];
-                        if (f & PF_ANGULAR) { ax = o[6]; ay = o[7]; az = o[8]; app = 2; }
-                    } else {
-                        jx = o[0]; jy = o[1]; jz = o[2];
-                        if (f & PF_ANGULAR) { ax = o[3]; ay = o[4]; az = o[5]; app = 2; }
-                    }
-                }
-            }
-            // only the entries that applied an impulse, in entry order (a wall's candidate list is
-            // long and few of its spheres touch it)
-            for (unsigned am = __ballot_sync(0xffffffffu, app != 0); am; am &= am - 1) {
-                const int q = __ffs(am) - 1;
-                const int a = __shfl_sync(0xffffffffu, app, q);
-                const double bx = __shfl_sync(0xffffffffu, jx, q), by = __shfl_sync(0xffffffffu, jy, q),
-                             bz = __shfl_sync(0xffffffffu, jz, q);
-                const double cx = __shfl_sync(0xffffffffu, ax, q), cy = __shfl_sync(0xffffffffu, ay, q),
-                             cz = __shfl_sync(0xffffffffu, az, q);
-                if (a) J = add(J, mk(bx, by, bz));
-                if (a == 2) JA = add(JA, mk(cx, cy, cz));
-            }
-        }
-    }
-    if (lane == 0)
-        finish_object(i, m, J, JA, dt, fimp, pos, vel, av, ox, oz, imp, aimp, write_imp, origin, pos32, wall32,
-                      ext_imp, ext_aimp, pb);
+    finish_object(i, m, J, JA, a.dt, a.fimp, a.pos, a.vel, a.av, a.ox, a.oz, a.imp, a.aimp, a.write_imp, a.origin,
+                  a.pos32, a.wall32, a.ext_imp, a.ext_aimp, a.pb);
 }
 
 // Narrow phase only: PF_ACTIVE of every pair at the current positions (the IsActive()
@@ -1449,18 +1473,30 @@ int Engine::step_once(bool write_impulses) {
     // AddFieldImpact + AddConstrainedImpact + Response (+ CheckContactStatus in the next k_pair_exact)
     const d3 fimp = muls(mk(g_[0], g_[1], g_[2]), dt);    // csp->GetFieldAcceleration() * dt (SimMediator.cpp:738)
     const d3 org = mk(origin_[0], origin_[1], origin_[2]);
-    k_obj<<<blocks_for(n_), TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_pos_, d_vel_, d_av_, d_ox_, d_oz_,
-                                               d_imp_, d_aimp_, cur_.csr_ptr, cur_.csr_ent, cur_.flags, cur_.out, dt,
-                                               fimp, write_impulses ? 1 : 0, org, d_pos32_, d_wall32_, ext_imp_, ext_aimp_,
-                                               tab_.pbc, d_touched_, d_nwork_);
+    ObjArgs oa;
+    oa.n = n_;
+    oa.model_of = d_model_of_;
+    oa.models = d_models_;
+    oa.pos = d_pos_; oa.vel = d_vel_; oa.av = d_av_; oa.ox = d_ox_; oa.oz = d_oz_; oa.imp = d_imp_; oa.aimp = d_aimp_;
+    oa.csr_ptr = cur_.csr_ptr;
+    oa.csr_ent = cur_.csr_ent;
+    oa.flags = cur_.flags;
+    oa.out = cur_.out;
+    oa.dt = dt;
+    oa.fimp = fimp;
+    oa.write_imp = write_impulses ? 1 : 0;
+    oa.origin = org;
+    oa.pos32 = d_pos32_;
+    oa.wall32 = d_wall32_;
+    oa.ext_imp = ext_imp_;
+    oa.ext_aimp = ext_aimp_;
+    oa.pb = tab_.pbc;
+    oa.touched = d_touched_;
+    oa.nwork = d_nwork_;
+    oa.nglob = (uint32_t)global_ids_.size();
+    oa.glob = d_global_;
+    k_obj<<<oa.nglob + blocks_for(n_), TPB, 0, stream_>>>(oa);
     ++launches_;
-    if (!global_ids_.empty()) {
-        k_obj_global<<<blocks_for((uint64_t)global_ids_.size() * 32), TPB, 0, stream_>>>(
-            (uint32_t)global_ids_.size(), d_global_, d_model_of_, d_models_, d_pos_, d_vel_, d_av_, d_ox_, d_oz_,
-            d_imp_, d_aimp_, cur_.csr_ptr, cur_.csr_ent, cur_.flags, cur_.out, dt, fimp, write_impulses ? 1 : 0, org,
-            d_pos32_, d_wall32_, ext_imp_, ext_aimp_, tab_.pbc, d_touched_);
-        ++launches_;
-    }
     if (prof) CK(cudaEventRecord(ev_[2], stream_));
     backup_pending_ = true;
     // NBSConsultant::NextStep (NBSConsultant.cpp:35-78)
