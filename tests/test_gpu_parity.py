@@ -418,3 +418,23 @@ def test_system_status_csv_matches_reference(case, engine_lib, tmp_path):
         assert fa[1:4] == fb[1:4], (a, b)                 # objects, records, contacts
         np.testing.assert_allclose([float(x) for x in fa], [float(x) for x in fb], rtol=1e-5, atol=1e-300,
                                    err_msg=f"{a} | {b}")
+
+
+@pytest.mark.parametrize("n_side,spacing", [(8, 2.4e-3), (12, 2.005e-3), (24, 2.005e-3), (34, 2.005e-3), (45, 2.005e-3)])
+def test_pair_kernel_candidates_per_block_bitexact(n_side, spacing, engine_lib, port_lib):
+    """The pair kernel at each of its block sizes (512, 1024 and 2048 candidates, remainders
+    included) and on a list of which it keeps nothing: 30 steps of colliding linear-law spheres with
+    rebuilds every 7, bit for bit against the oracle."""
+    from oracle import PortWorld
+    sc = scenes.lsd_box(n_side=n_side, steps=400, spacing=spacing, vel_sigma=0.3, box_width=n_side * spacing + 1e-3,
+                        box_height=n_side * spacing + 5e-3)
+    e = engine_lib.GpuEngine(sc, up_iact=7)
+    p = PortWorld(sc, up_iact=7)
+    e.run(30)
+    p.run(30)
+    a, b = e.state(), p.state()
+    for k in ("position", "velocity", "angular_velocity", "impact", "angular_impact"):
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+    ia, ib = e.interactions(), p.interactions()
+    assert np.array_equal(ia["active"], ib["active"].astype(np.uint8))
+    e.close()
