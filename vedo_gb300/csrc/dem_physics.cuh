@@ -261,9 +261,9 @@ __device__ __forceinline__ void respond_object(const ModelDev& m, double dt, d3 
         d3 dp = smul(dt, add(V, smul(0.5, dv)));
         d3 dw = smul(dt, add(AV, smul(0.5, dav)));
         P = add(P, dp);
-        const Turn T = turn_of(dw);
-        Ox = rotate_by(Ox, T);
-        Oz = rotate_by(Oz, T);
+        const Turn T = sphere_turn(dw);
+        Ox = sphere_rotate(Ox, T);
+        Oz = sphere_rotate(Oz, T);
         V = add(V, dv);
         AV = add(AV, dav);
     } else if (m.behavior == BEH_ORBITAL) {                   // DOOrbitalQuasiPlate.cpp:18-34

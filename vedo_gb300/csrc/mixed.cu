@@ -1023,9 +1023,9 @@ __device__ __forceinline__ void turn_sphere(const TickArgs& a, uint32_t i) {
     const d3 W2 = ld(a.w64, i);
     const d3 dwv = smul(S.dt, sub(W2, smul(0.5, mk(f2d(dav.x), f2d(dav.y), f2d(dav.z)))));
     if (dwv.x == 0.0 && dwv.y == 0.0 && dwv.z == 0.0) return;
-    const Turn T = turn_of(dwv);
-    st(a.sox, i, rotate_by(ld(a.sox, i), T), 0.0);
-    st(a.soz, i, rotate_by(ld(a.soz, i), T), 0.0);
+    const Turn T = sphere_turn(dwv);
+    st(a.sox, i, sphere_rotate(ld(a.sox, i), T), 0.0);
+    st(a.soz, i, sphere_rotate(ld(a.soz, i), T), 0.0);
 }
 __global__ void __launch_bounds__(TPB) k_turn(TickArgs a) {
     step_order();
