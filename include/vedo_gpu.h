@@ -157,7 +157,8 @@ typedef struct vedo_engine_opts {
                                  travel together may have used that up                  */
     uint32_t check_interval;  /* MIXED only: steps between displacement checks (10)   */
     uint32_t tick_block;      /* MIXED only: threads per block of the tick kernel, 32..256,
-                                 a multiple of 32 (0 = 256)                            */
+                                 a multiple of 32 (0 = 256); a scene too small to give every
+                                 SM a block takes smaller ones                          */
     float cell_scale;         /* MIXED only: cell edge as a multiple of 2 r_max + skin,
                                  >= 1 (0 = 1)                                          */
     uint32_t autotune;        /* MIXED only: 1 = the first steps of the run choose the tick

@@ -386,3 +386,44 @@ def test_plate_with_circular_hole_mixed_against_fp64(engine_lib, tmp_path):
     b.run(1)
     sa, sb = a.state(("impact",)), b.state(("impact",))
     assert np.linalg.norm(sa["impact"] - sb["impact"]) <= 1e-5 * np.linalg.norm(sa["impact"])
+
+
+@pytest.mark.parametrize("n,block", [(300, 32), (2000, 256), (9000, 64), (15000, 96), (30000, 128), (60001, 256),
+                                     (90000, 192)])
+@pytest.mark.parametrize("stored", [False, True])
+def test_tick_threads_per_sphere_agree_with_the_pair_pass(n, block, stored, engine_lib):
+    """The full tick at 8, 4, 2 and 1 threads a sphere and odd block sizes: hoppers draining (wall and
+    sphere pairs), against the pair pass, whose kernels are others: identical bits."""
+    sc = scenes.hopper(n=n, seed=n, steps=1000, touching=True)
+    sc.velocity[:n] = np.random.default_rng(n).normal(0.0, 0.05, size=(n, 3))
+    a = engine_lib.GpuEngine(sc, precision=1, tick_block=block, stored_splits=stored)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True)
+    for k in (1, 29):
+        a.run(k)
+        b.run(k)
+        _same_run(a, b)
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("big", [0.0, 6e-3])
+@pytest.mark.parametrize("n", [1500, 12000, 40000])
+def test_tick_with_more_pairs_than_its_slots(n, big, engine_lib):
+    """A packing (twelve pairs on the exact path a sphere: more than the block's shared slots hold at
+    once), and one with a sphere several times larger in it, whose list is longer than 64 entries: the
+    full tick against the pair pass, identical bits."""
+    sc = scenes.dense_pack(n=n, steps=1000)
+    if big:
+        import copy
+        sc.models = list(sc.models) + [copy.deepcopy(sc.models[0])]
+        sc.models[-1].name, sc.models[-1].attrs = "Big", (big,)
+        sc.model_index[n // 2] = len(sc.models) - 1
+        sc.position[n // 2, 2] = sc.position[:n, 2].max() + 0.9 * big
+    a = engine_lib.GpuEngine(sc, precision=1)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True)
+    for k in (1, 9):
+        a.run(k)
+        b.run(k)
+        _same_run(a, b)
+    a.close()
+    b.close()

@@ -573,20 +573,22 @@ __device__ __noinline__ bool clean_history(const TickArgs& a, uint32_t e, uint8_
 // the pairs that are certainly apart (rebuild-time distance minus both spheres' travel since
 // then): their history is cleaned and their wall-impulse share zeroed.  Returns the mask of
 // entries that need the exact path.  The side effects are idempotent, so a walk that is
-// abandoned and redone (the split tick) leaves the same state.
+// abandoned and redone (the split tick) leaves the same state.  The group's entries are `step`
+// apart (a sphere walked by several lanes).
 template <bool PBC>
 __device__ __forceinline__ uint32_t prefilter_group(const TickArgs& a, uint32_t base, uint32_t e1, const float4& p32i,
                                                     float pad, bool& dirty, uint32_t& owned, uint32_t& walls,
-                                                    const float* L) {
+                                                    const float* L, uint32_t step = 1u) {
     uint32_t ge[TICK_GROUP], gm[TICK_GROUP];
     uint8_t gf[TICK_GROUP];
     float4 gp[TICK_GROUP];
 #pragma unroll
     for (int k = 0; k < TICK_GROUP; ++k) {
-        const bool ok = base + k < e1;
-        ge[k] = ok ? a.nent[base + k] : 0u;
-        gm[k] = ok ? a.nmeta[base + k] : 0u;     // cd 0: nothing to do
-        gf[k] = ok ? a.fA[base + k] : (uint8_t)0;
+        const uint32_t e = base + (uint32_t)k * step;
+        const bool ok = e < e1;
+        ge[k] = ok ? a.nent[e] : 0u;
+        gm[k] = ok ? a.nmeta[e] : 0u;     // cd 0: nothing to do
+        gf[k] = ok ? a.fA[e] : (uint8_t)0;
     }
 #pragma unroll
     for (int k = 0; k < TICK_GROUP; ++k)
@@ -597,7 +599,7 @@ __device__ __forceinline__ uint32_t prefilter_group(const TickArgs& a, uint32_t 
         const uint32_t meta = gm[k];
         const int cd = (int)((meta >> META_CD_SHIFT) & META_CD_MASK);
         if (cd == 0) continue;
-        const uint32_t e = base + k;
+        const uint32_t e = base + (uint32_t)k * step;
         const uint32_t j = ge[k] & ~WALL_BIT;
         const bool wall = ge[k] & WALL_BIT;
         const bool i_slave = meta & META_SLAVE;
@@ -633,9 +635,9 @@ __device__ __forceinline__ uint32_t prefilter_group(const TickArgs& a, uint32_t 
 // (a separate instance: the common path carries none of it).
 __device__ __forceinline__ uint32_t prefilter_any(const TickArgs& a, uint32_t base, uint32_t e1, const float4& p32i,
                                                   float pad, bool& dirty, uint32_t& owned, uint32_t& walls,
-                                                  const float* L) {
-    return L ? prefilter_group<true>(a, base, e1, p32i, pad, dirty, owned, walls, L)
-             : prefilter_group<false>(a, base, e1, p32i, pad, dirty, owned, walls, nullptr);
+                                                  const float* L, uint32_t step = 1u) {
+    return L ? prefilter_group<true>(a, base, e1, p32i, pad, dirty, owned, walls, L, step)
+             : prefilter_group<false>(a, base, e1, p32i, pad, dirty, owned, walls, nullptr, step);
 }
 
 // Quiet spheres.  Between rebuilds a sphere's list, the rebuild-time positions and the fixed
@@ -919,16 +921,175 @@ __device__ __forceinline__ void step_order() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The full tick, one thread per sphere.
+// The full tick: a block takes blockDim / 2^lanes spheres.  A sphere's list is prefiltered by 2^lanes
+// threads side by side; the block's entries on the exact path then go to its threads one entry each,
+// the sphere pairs from the first thread up and the wall pairs (FP64 detectors) from the last down, so
+// that the two run in warps of their own; each entry's share is left in shared memory, and one thread
+// per sphere adds its shares in entry order and integrates.  Every pair's and every sphere's
+// operations are tick_sphere's, in its order, so the bits are the same however the work is spread.
+// What bounds a small scene is latency, not work: a thread that walks its sphere's list and then
+// evaluates the pairs one after the other takes 2 to 10 us for each while most of the GPU idles.  With
+// one pair a thread a 2,000-sphere hopper's step went from 89 to 27 us and the settling 8,000-sphere
+// box's from 67 to 24; the 60,000-sphere hopper's from 103 to 60 and 20,000 packed spheres' from 89 to
+// 55 us (no lane waits for the sphere of its warp with the most pairs).
+constexpr uint32_t SHARES_PER_SPHERE = 6;     // shared-memory slots a block holds at once, per sphere
+__host__ __device__ __forceinline__ uint32_t tick_slots(uint32_t spheres) {
+    return spheres * SHARES_PER_SPHERE > 64u ? spheres * SHARES_PER_SPHERE : 64u;   // at least one sphere's chunk
+}
+template <int LAW, bool XS, int KIND>
+__device__ __forceinline__ void tick_item(const TickArgs& a, uint32_t base, const uint2& it, float4* share) {
+    const uint32_t e = it.x, i = base + (it.y >> 16), slot = it.y & 0xffffu;
+    const uint32_t meta = a.nmeta[e];
+    const d3 Pi = XS || KIND == 2 ? mk(0.0, 0.0, 0.0) : ld(a.xA, i);
+    f3 Jp, tA, tB;
+    const int app = exact_pair<LAW, XS, KIND>(a, a.scenes[a.scene_of[i]], i, Pi, e, a.nent[e], meta, Jp, tA, tB);
+    const bool i_slave = meta & META_SLAVE;
+    const f3 Ji = i_slave ? Jp : -Jp, ti = i_slave ? tA : tB;
+    share[2 * slot] = make_float4(Ji.x, Ji.y, Ji.z, __int_as_float(app));
+    share[2 * slot + 1] = make_float4(ti.x, ti.y, ti.z, 0.0f);
+}
 template <int LAW, bool XS>
-__global__ void __launch_bounds__(TPB) k_tick(TickArgs a) {
+__global__ void __launch_bounds__(TPB, 2) k_tick(TickArgs a, int lanes) {
+    extern __shared__ float4 share[];              // [2 * slots], then the slots' items
+    __shared__ uint32_t pk[TPB + 1], warp_tot[TPB / 32];
+    __shared__ uint8_t note[TPB];                  // per sphere: 1 stepped, 2 quiet, 4 frozen, 8 no clean walk, count << 4
     step_order();
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = threadIdx.x, B = blockDim.x >> lanes, G = 1u << lanes;
+    const uint32_t s = t >> lanes, g = t & (G - 1u), base = blockIdx.x * B;
+    if (held_step(a)) {                            // the same value for every thread of the launch
+        if (t < B) hold_state(a, base + t);
+        return;
+    }
+    const uint32_t slots = tick_slots(B);
+    uint2* items = reinterpret_cast<uint2*>(share + 2 * slots);
+    const int lane = (int)(t & 31u);
+    uint32_t c0 = 0u, e1 = 0u;
+    float4 p32i = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float pad = 0.0f;
+    const float* L = nullptr;
+    bool walk = false, reset = false;
+    {
+        const uint32_t i = base + s;
+        uint8_t nt = 0;
+        if (i < a.n) {
+            const ModelDev& M = a.models[a.model_of[i]];
+            const SceneDev& S = a.scenes[a.scene_of[i]];
+            if (M.scope == SCOPE_LOCAL && S.active) {
+                const uint32_t qc = a.qcnt[i];
+                const float2 cl = a.clear[i];
+                pad = 2.0f * a.disp[0];
+                const bool quiet = qc >= 2u && !a.write_imp && pad <= cl.x && a.disp[1] <= cl.y;
+                nt = (uint8_t)(1u | (quiet ? 2u : 0u) | qc << 4);
+                if (!quiet) {
+                    c0 = a.nptr[i];
+                    e1 = a.nptr[i + 1];
+                    p32i = a.pos32[i];
+                    if (S.pb.on) L = S.pb.range32;
+                    walk = true;
+                }
+            } else if (M.scope == SCOPE_LOCAL) {
+                nt = 4u;                           // a finished scene waits, unchanged
+            }
+        }
+        if (g == 0u) note[s] = nt;
+    }
+    K3 J, JA;                                      // (of sphere t, in the first B threads)
+    // The lists are walked in chunks of 64 entries (one chunk for nearly every sphere)
+    for (;;) {
+        const bool more = walk && c0 < e1;
+        if (!__syncthreads_or(more)) break;
+        unsigned long long mine = 0ull, wmine = 0ull;      // this thread's entries on the exact path
+        if (more) {
+            const uint32_t c1 = min(e1, c0 + 64u);
+            for (uint32_t k0 = g; c0 + k0 < c1; k0 += TICK_GROUP * G) {
+                uint32_t owned = 0u, walls = 0u;           // (owned: unused here)
+                const uint32_t m = prefilter_any(a, c0 + k0, c1, p32i, pad, reset, owned, walls, L, G);
+#pragma unroll
+                for (uint32_t u = 0; u < TICK_GROUP; ++u) {
+                    mine |= (unsigned long long)((m >> u) & 1u) << ((k0 + u * G) & 63u);
+                    wmine |= (unsigned long long)((walls >> u) & 1u) << ((k0 + u * G) & 63u);
+                }
+            }
+        }
+        unsigned long long full = mine, wfull = wmine;     // the sphere's
+        for (uint32_t o = 1u; o < G; o <<= 1) {
+            full |= __shfl_xor_sync(0xffffffffu, full, (int)o);
+            wfull |= __shfl_xor_sync(0xffffffffu, wfull, (int)o);
+        }
+        reset |= full != 0ull;
+        // exclusive prefixes over the block's spheres: sphere pairs in the low half, wall pairs in the high
+        const uint32_t own = g == 0u ? (uint32_t)__popcll(full & ~wfull) | (uint32_t)__popcll(wfull) << 16 : 0u;
+        uint32_t incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) warp_tot[t >> 5] = incl;
+        __syncthreads();
+        uint32_t before = 0u;
+        for (uint32_t w = 0; w < t >> 5; ++w) before += warp_tot[w];
+        if (g == 0u) pk[s] = before + incl - own;
+        if (t == blockDim.x - 1u) pk[B] = before + incl;
+        __syncthreads();
+        auto slot_of = [&](uint32_t q) { return (pk[q] & 0xffffu) + (pk[q] >> 16); };
+        // as many whole spheres at a time as the slots hold (nearly always all)
+        for (uint32_t s0 = 0u; s0 < B;) {
+            const uint32_t first = slot_of(s0), P0 = pk[s0] & 0xffffu, W0 = pk[s0] >> 16;
+            uint32_t s1 = B;
+            if (slot_of(B) - first > slots) {
+                uint32_t lo = s0 + 1u, hi = B;     // the last s1 whose spheres fit (one always does)
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi + 1u) >> 1;
+                    if (slot_of(mid) - first <= slots) lo = mid; else hi = mid - 1u;
+                }
+                s1 = lo;
+            }
+            const uint32_t nP = (pk[s1] & 0xffffu) - P0, nW = (pk[s1] >> 16) - W0;
+            if (s >= s0 && s < s1)
+                for (unsigned long long b = mine; b; b &= b - 1ull) {
+                    const int k = __ffsll((long long)b) - 1;
+                    const unsigned long long below = (1ull << k) - 1ull;
+                    const uint32_t at = (wfull >> k) & 1ull
+                                            ? nP + (pk[s] >> 16) - W0 + (uint32_t)__popcll(wfull & below)
+                                            : (pk[s] & 0xffffu) - P0 + (uint32_t)__popcll(full & ~wfull & below);
+                    items[at] = make_uint2(c0 + (uint32_t)k,
+                                           s << 16 | (slot_of(s) - first + (uint32_t)__popcll(full & below)));
+                }
+            __syncthreads();
+            for (uint32_t q = t; q < nP; q += blockDim.x) tick_item<LAW, XS, 1>(a, base, items[q], share);
+            for (uint32_t q = blockDim.x - 1u - t; q < nW; q += blockDim.x)
+                tick_item<LAW, XS, 2>(a, base, items[nP + q], share);
+            __syncthreads();
+            if (t >= s0 && t < s1)
+                for (uint32_t q = slot_of(t) - first; q < slot_of(t + 1u) - first; ++q) {
+                    const float4 r0 = share[2 * q];
+                    const int app = __float_as_int(r0.w);
+                    if (app) {
+                        J.add(f4to3(r0));
+                        if (app == 2) JA.add(f4to3(share[2 * q + 1]));
+                    }
+                }
+            s0 = s1;
+            if (s0 < B) __syncthreads();           // (the chunk's end: the loop's barrier)
+        }
+        c0 += 64u;
+    }
+    for (uint32_t o = 1u; o < G; o <<= 1) reset |= __shfl_xor_sync(0xffffffffu, (int)reset, (int)o) != 0;
+    if (g == 0u && reset) note[s] |= 8u;
+    __syncthreads();
     float2 vmax_local = make_float2(0.0f, 0.0f);
-    if (held_step(a)) {                          // the same value for every thread of the launch
-        hold_state(a, t);
-    } else if (t < a.n) {
-        vmax_local = tick_sphere<LAW, XS>(a, t);
+    if (t < B) {
+        const uint32_t i = base + t, nt = note[t];
+        if (nt & 1u) {
+            const bool quiet = nt & 2u;
+            const uint32_t mi = a.model_of[i];
+            if (!quiet) note_walk(a, i, nt >> 4, nt & 8u);
+            vmax_local = finish_sphere<XS>(a, i, a.models[mi].behavior == BEH_MOBILE, quiet, a.scenes[a.scene_of[i]],
+                                           ld(a.xA, i), ld(a.v64, i), a.mf[2 * mi], a.mf[2 * mi + 1], J, JA);
+        } else if (nt & 4u) {
+            hold_state(a, i);
+        }
     }
     reduce_vmax(a, vmax_local);
 }
@@ -2691,6 +2852,7 @@ private:
     }
     int rebuild();
     void launch_step(bool write_imp);
+    cudaError_t launch_tick(bool dep, void (*k)(TickArgs, int), const TickArgs& a);
     cudaError_t launch_err_ = cudaSuccess;   // the first failed launch of the step kernels
     int step_chunk(uint32_t chunk, bool imp_last, float* use_after);
     int autotune(uint32_t max_steps, uint32_t* taken);
@@ -3641,11 +3803,12 @@ int MixedEngine::rebuild() {
 // A per-step kernel launch; `dep`: with programmatic dependent launch (the kernel orders itself
 // after the previous one with step_order()).
 template <typename... P, typename... A>
-static cudaError_t step_launch(bool dep, void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A... args) {
+static cudaError_t step_launch_smem(bool dep, void (*k)(P...), unsigned grid, unsigned block, size_t smem,
+                                    cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -3653,6 +3816,31 @@ static cudaError_t step_launch(bool dep, void (*k)(P...), unsigned grid, unsigne
     cfg.attrs = at;
     cfg.numAttrs = dep ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, k, args...);
+}
+template <typename... P, typename... A>
+static cudaError_t step_launch(bool dep, void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A... args) {
+    return step_launch_smem(dep, k, grid, block, 0, s, args...);
+}
+
+// The full tick's launch.  Threads per sphere: 8 or 4 while that keeps every sphere of the scene resident
+// at once (512 threads an SM at the tick's registers), 2 up to two rounds of that, then 1.  us per step
+// at 1 / 2 / 4 / 8 (GB300): 8,000-sphere box 37 / 29 / 26 / 24; 10,000 loose spheres 12 / 12 / 12 / 14;
+// 20,000 packed 71 / 55 / 64 / 69; 40,000-sphere drum 39 / 34 / 36 / 44; 60,000-sphere hopper 74 / 60 /
+// 73 / 102; 200,000 packed 224 / 257 / 350 / 485.  A scene that leaves SMs without a block takes smaller
+// blocks than tick_block, down to 64 threads (2,000-sphere hopper, 256 to 64: 35 to 27).
+cudaError_t MixedEngine::launch_tick(bool dep, void (*k)(TickArgs, int), const TickArgs& a) {
+    const uint64_t room = (uint64_t)sms_ * 512u;
+    int lanes = n_ <= room ? 1 : 0;
+    while (lanes >= 1 && lanes < 3 && ((uint64_t)n_ << (lanes + 1)) <= room) ++lanes;
+    unsigned block = (unsigned)tpb_;
+    while (block >= 128u && block % 64u == 0u && ((uint64_t)n_ << lanes) < (uint64_t)sms_ * block) block /= 2u;
+    const unsigned spheres = block >> lanes;
+    const size_t bytes = (size_t)tick_slots(spheres) * (2 * sizeof(float4) + sizeof(uint2));
+    if (bytes > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+    }
+    return step_launch_smem(dep, k, (n_ + spheres - 1u) / spheres, block, bytes, stream_, a, lanes);
 }
 
 void MixedEngine::launch_step(bool write_imp) {
@@ -3713,9 +3901,11 @@ void MixedEngine::launch_step(bool write_imp) {
         nb_full = std::min<unsigned>(nb, (unsigned)sms_ * 512u / (unsigned)tpb_);
     }
 #define VEDO_TICK(L)                                                                                        \
-    note(step_launch(dep, split_tick_ ? (xs_stored_ ? k_tick_work<L, true> : k_tick_work<L, false>)          \
-                                      : (xs_stored_ ? k_tick<L, true> : k_tick<L, false>),                   \
-                     split_tick_ ? nb_full : nb, (unsigned)tpb_, stream_, a))
+    if (split_tick_)                                                                                        \
+        note(step_launch(dep, xs_stored_ ? k_tick_work<L, true> : k_tick_work<L, false>, nb_full,            \
+                         (unsigned)tpb_, stream_, a));                                                       \
+    else                                                                                                    \
+        note(launch_tick(dep, xs_stored_ ? k_tick<L, true> : k_tick<L, false>, a))
     switch (law_) {
     case IS_BSDBF: VEDO_TICK(IS_BSDBF); break;
     case IS_BTSDBF: VEDO_TICK(IS_BTSDBF); break;
