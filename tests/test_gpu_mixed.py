@@ -427,3 +427,20 @@ def test_tick_with_more_pairs_than_its_slots(n, big, engine_lib):
         _same_run(a, b)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,block", [(70000, 32), (70000, 256), (450000, 64)])
+def test_pair_worklists_handed_out_in_chunks(n, block, engine_lib):
+    """Worklists longer than the pair kernels' grids, which the warps take chunk by chunk (one round
+    of pairs a chunk, and several): a dense packing against the full tick, identical bits."""
+    sc = scenes.dense_pack(n=n, steps=1000)
+    a = engine_lib.GpuEngine(sc, precision=1)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True, tick_block=block)
+    for k in (1, 11):
+        a.run(k)
+        b.run(k)
+        sa, sb = a.state(), b.state()
+        for f in ("position", "velocity", "angular_velocity", "impact", "angular_impact"):
+            assert np.array_equal(sa[f], sb[f]), f
+    a.close()
+    b.close()

@@ -467,6 +467,7 @@ struct TickArgs {
     uint32_t* work;                // split tick: spheres deferred to the full tick (else nullptr)
     uint32_t* nwork;               // split tick: spheres in `work`; pair pass: sphere pairs in `pwork`
                                    // (from its start), and nwork[-1] wall pairs (from its end)
+    uint32_t* taken;               // pair pass: chunks taken of the sphere pairs, and [1] of the wall pairs
     uint4* pwork;                  // pair pass: (owner entry, its sphere, entry word, meta word) of every
                                    // pair on the exact path
     uint8_t* xf;                   // pair pass: [ne] 1 = the entry is on the exact path this step
@@ -754,6 +755,19 @@ __device__ __forceinline__ int exact_pair(const TickArgs& a, const SceneDev& S, 
     bool active;
     float depth;
     f3 n, rA, rB;
+    uint8_t f0;
+    float4 h, vs4, vm4, ws4, wm4;
+    if (KIND == 1) {
+        // every gather of the pair issued together: after the overlap's tie branch (a call) the
+        // velocities and the history waited for a second and a third round of latency (1,000,000
+        // packed spheres: 526 to 508 us a step)
+        f0 = a.fA[slot];
+        h = a.hA[slot];
+        vs4 = a.v32A[s];
+        vm4 = a.v32A[m];
+        ws4 = a.w32A[s];
+        wm4 = a.w32A[m];
+    }
     if (KIND == 1 || (KIND == 0 && P.cd == CD_SS)) {
         // d = x_master - x_slave, |d|^2 and R^2 - |d|^2 in double-float from the two
         // positions' hi/lo splits; where the numerator is within 1e-9 R^2 of zero the
@@ -800,14 +814,22 @@ __device__ __forceinline__ int exact_pair(const TickArgs& a, const SceneDev& S, 
     } else if (KIND != 1) {
         wall_pair(a, P.cd, pi, s, m, active, depth, n, rA, rB, S.pb);
     }
-    const uint8_t f0 = a.fA[slot];
+    if (KIND != 1) {
+        f0 = a.fA[slot];
+        h = ((f0 & 15) != 0 || active) ? a.hA[slot] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        vs4 = a.v32A[s];
+        vm4 = a.v32A[m];
+        ws4 = a.w32A[s];
+        wm4 = a.w32A[m];
+    } else if ((f0 & 15) == 0 && !active) {
+        h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
     uint8_t f = f0 & 15;
-    float4 h = (f != 0 || active) ? a.hA[slot] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     Jp = fm(0.0f, 0.0f, 0.0f);
     tA = Jp;
     tB = Jp;
-    const int app = solve32<LAW>(P.is, a.pc32 + 8 * (size_t)pi, active, depth, n, rA, rB, f4to3(a.v32A[s]),
-                                 f4to3(a.v32A[m]), f4to3(a.w32A[s]), f4to3(a.w32A[m]), dtf, f, h, Jp, tA, tB);
+    const int app = solve32<LAW>(P.is, a.pc32 + 8 * (size_t)pi, active, depth, n, rA, rB, f4to3(vs4),
+                                 f4to3(vm4), f4to3(ws4), f4to3(wm4), dtf, f, h, Jp, tA, tB);
     if (e == slot) {                           // history owner writes the new status
         if (f != 0 || (f0 & 15) != 0) {
             a.hB[slot] = h;
@@ -1365,22 +1387,53 @@ __device__ __forceinline__ void pairs_from(const TickArgs& a, uint32_t first, ui
         for (uint32_t q = first; q < nww; q += stride) pair_item<LAW, XS, 2>(a, a.pwork[a.pcap - 1u - q]);
     }
 }
+// The same with the long worklists handed out as the warps ask for more: with a share per block fixed at
+// launch, the sphere-pair blocks that found no room beside the wall-pair kernel began theirs when the
+// others ended (700,000 spheres in 48 hoppers: 445 us a step with the two kernels side by side, 355 one
+// after the other, 320 like this; 1,000,000 packed spheres 508 to 480).  A list of at most a pair a thread is taken as it lies: every warp
+// asking at once costs about 1 ns each on the one counter (60,000-sphere hopper: 47 us a step so, 57
+// asking).  Longer ones go in about eight chunks a warp, the first of the blocks that surely start at
+// once fixed, the next one asked for before the present one is worked on.
+template <int LAW, bool XS, int KIND>
+__device__ __forceinline__ void pairs_taken(const TickArgs& a) {
+    const uint32_t nw = min(a.nwork[0], a.pcap), count = KIND == 1 ? nw : min(a.nwork[-1], a.pcap - nw);
+    const uint32_t threads = gridDim.x * blockDim.x;
+    auto item = [&](uint32_t q) { pair_item<LAW, XS, KIND>(a, a.pwork[KIND == 1 ? q : a.pcap - 1u - q]); };
+    if (count <= threads) {
+        const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+        if (q < count) item(q);
+        return;
+    }
+    const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5, given = gridDim.x / 2u * wpb;
+    const uint32_t chunk = max(1u, count / (threads * 8u)) * 32u;
+    uint32_t* const ctr = a.taken + (KIND == 1 ? 0 : 1);
+    auto ask = [&]() { return lane == 0u ? given + atomicAdd(ctr, 1u) : 0u; };
+    const uint32_t gw = blockIdx.x * wpb + (threadIdx.x >> 5);
+    uint32_t c = gw < given ? gw : __shfl_sync(0xffffffffu, ask(), 0);
+    while ((uint64_t)c * chunk < count) {
+        const uint32_t next = ask();
+        const uint32_t end = min(c * chunk + chunk, count);
+        for (uint32_t q = c * chunk + lane; q < end; q += 32u) item(q);
+        __syncwarp();
+        c = __shfl_sync(0xffffffffu, next, 0);
+    }
+}
 // AFTER_WALLS: launched after the wall-pair kernel, whose blocks all waited for the prefilter pass
 // before releasing this one, so the worklist is complete when it starts; it waits for the
 // wall-pair kernel only at its end, so that the two run side by side (the wall pairs' FP64 work
 // and the sphere pairs' gathers use different units), and the sum kernel after it, waiting for
 // it, then waits for both.
 template <int LAW, bool XS, int KIND, bool AFTER_WALLS>
-__global__ void __launch_bounds__(TPB, 4) k_tick_pairs(TickArgs a) {     // sphere pairs: 56 registers, no spills
+__global__ void __launch_bounds__(TPB, 4) k_tick_pairs(TickArgs a) {     // sphere pairs: 64 registers, no spills
     if (AFTER_WALLS) {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        if (!held_step(a)) pairs_from<LAW, XS, KIND>(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+        if (!held_step(a)) pairs_taken<LAW, XS, KIND>(a);
         asm volatile("griddepcontrol.wait;" ::: "memory");
         return;
     }
     step_order();
     if (held_step(a)) return;
-    pairs_from<LAW, XS, KIND>(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    pairs_taken<LAW, XS, KIND>(a);
 }
 
 // One sphere's sums and integration (or, in an identity step, its state carried over); returns its
@@ -1529,6 +1582,7 @@ struct WallArgs {
     unsigned* held;
     float4* wall32;
     unsigned* nwork;
+    unsigned* taken;
     const double4_32a* imp;
     const double4_32a* aimp;
     unsigned* dyn_bits;
@@ -1561,12 +1615,14 @@ __device__ __forceinline__ void walls_item(const WallArgs& W, uint32_t q) {
     unsigned* held = W.held;
     float4* wall32 = W.wall32;
     unsigned* nwork = W.nwork;
+    unsigned* taken = W.taken;
     const double4_32a* imp = W.imp;
     const double4_32a* aimp = W.aimp;
     unsigned* dyn_bits = W.dyn_bits;
     const float drel = disp_in[0], dabs = disp_in[1], dw = disp_in[2];
     const bool hold = list_spent(drel, dabs, dw, skin, skin_w);
     if (q == 0) {
+        taken[0] = taken[1] = 0u;
         nwork[0] = nwork[1] = 0u;                  // the worklists' counts (pair pass: wall pairs, then
                                                    // sphere pairs and the split tick's spheres), empty
                                                    // for the next step
@@ -3337,12 +3393,12 @@ int MixedEngine::init_from(const std::vector<SceneSource>& src, const MixedEngin
     }
     MCK(mal(&d_v64_, n_)); MCK(mal(&d_w64_, n_)); MCK(mal(&d_ox_, n_)); MCK(mal(&d_oz_, n_));
     MCK(mal(&d_imp_, n_)); MCK(mal(&d_aimp_, n_)); MCK(mal(&d_pos32_, n_)); MCK(mal(&d_wall32_, n_));
-    MCK(mal(&d_red_, 16)); MCK(mal(&d_disp_, 8)); MCK(mal(&d_err_, 1));
+    MCK(mal(&d_red_, 18)); MCK(mal(&d_disp_, 8)); MCK(mal(&d_err_, 1));
     MCK(mal(&d_key_, n_)); MCK(mal(&d_key_alt_, n_)); MCK(mal(&d_sid_, n_)); MCK(mal(&d_sid_alt_, n_));
     MCK(mal(&d_cnt_, (size_t)n_ + 1));
     MCK(mal(&d_stage_, 7 * 3 * (size_t)n_));
     MCK(mal(&d_obs_, (size_t)(nblk(n_) + 2) * 16 + 64));
-    MCK(cudaMemset(d_red_, 0, 64));
+    MCK(cudaMemset(d_red_, 0, 72));
     MCK(cudaMemset(d_disp_, 0, 32));
     if (prev) {
         for (int k = 0; k < 3; ++k) origin_[k] = prev->origin_[k];
@@ -3491,6 +3547,7 @@ WallArgs MixedEngine::wargs(int c) {
     w.held = d_red_ + 11;
     w.wall32 = d_wall32_;
     w.nwork = d_red_ + 13;
+    w.taken = d_red_ + 16;
     w.imp = d_imp_;
     w.aimp = d_aimp_;
     w.dyn_bits = d_red_ + 3;
@@ -3547,6 +3604,7 @@ TickArgs MixedEngine::args(bool write_imp) {
     a.xs_stored = xs_stored_ ? 1 : 0;
     a.work = split_tick_ ? d_work_ : nullptr;
     a.nwork = d_red_ + 14;
+    a.taken = d_red_ + 16;
     a.pwork = d_pwork_;
     a.xf = d_xf_;
     a.prec = d_prec_;
