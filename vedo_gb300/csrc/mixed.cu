@@ -1586,144 +1586,145 @@ struct WallArgs {
     const double4_32a* imp;
     const double4_32a* aimp;
     unsigned* dyn_bits;
+    int dyn;                       // a wall responds to its impulses (mobile or constrained)
 };
-__device__ __forceinline__ void walls_item(const WallArgs& W, uint32_t q) {
-    const uint32_t nglob = W.nglob;
-    const uint32_t* __restrict__ glob = W.glob;
-    const uint32_t* __restrict__ model_of = W.model_of;
-    const ModelDev* __restrict__ models = W.models;
-    const SceneDev* __restrict__ scenes = W.scenes;
-    const uint32_t* __restrict__ scene_of = W.scene_of;
-    const double4_32a* xA = W.xA;
-    double4_32a* xB = W.xB;
-    double4_32a* v64 = W.v64;
-    double4_32a* w64 = W.w64;
-    const float4* v32A = W.v32A;
-    float4* v32B = W.v32B;
-    const float4* w32A = W.w32A;
-    float4* w32B = W.w32B;
-    double4_32a* ox = W.ox;
-    double4_32a* oz = W.oz;
-    const float dt_max = W.dt_max;
-    unsigned* vmax_bits = W.vmax_bits;
-    unsigned* vrel_bits = W.vrel_bits;
-    const float* disp_in = W.disp_in;
-    float* disp_out = W.disp_out;
-    const float skin = W.skin, skin_w = W.skin_w, pos_eps = W.pos_eps;
-    const unsigned* wall_speed_bits = W.wall_speed_bits;
-    const double4_32a* __restrict__ wrot = W.wrot;
-    unsigned* held = W.held;
-    float4* wall32 = W.wall32;
-    unsigned* nwork = W.nwork;
-    unsigned* taken = W.taken;
-    const double4_32a* imp = W.imp;
-    const double4_32a* aimp = W.aimp;
-    unsigned* dyn_bits = W.dyn_bits;
-    const float drel = disp_in[0], dabs = disp_in[1], dw = disp_in[2];
-    const bool hold = list_spent(drel, dabs, dw, skin, skin_w);
-    if (q == 0) {
-        taken[0] = taken[1] = 0u;
-        nwork[0] = nwork[1] = 0u;                  // the worklists' counts (pair pass: wall pairs, then
-                                                   // sphere pairs and the split tick's spheres), empty
-                                                   // for the next step
-        if (hold) {
-            for (int k = 0; k < 4; ++k) disp_out[k] = disp_in[k];
-            *held += 1u;
-        } else {
-            // pos_eps: the FP64 rounding of a position update, which the speeds do not see
-            disp_out[0] = drel + dt_max * __uint_as_float(*vrel_bits) + pos_eps;
-            disp_out[1] = dabs + dt_max * __uint_as_float(*vmax_bits) + pos_eps;
-            disp_out[2] = dw + dt_max * __uint_as_float(*wall_speed_bits) + pos_eps;
-            disp_out[3] = __uint_as_float(__float_as_uint(disp_in[3]) + 1u);
-        }
-        *vmax_bits = 0u;
-        *vrel_bits = 0u;
-    }
-    if (q >= nglob) return;
-    const uint32_t w = glob[q];
-    if (hold || !scenes[scene_of[w]].active) {
-        xB[w] = xA[w];
-        v32B[w] = v32A[w];
-        w32B[w] = w32A[w];
-        return;
-    }
-    const ModelDev& M = models[model_of[w]];
-    const SceneDev& S = scenes[scene_of[w]];
+// A wall's next state, from its present one and (a responding wall) its impulses of the step.
+struct WallStep {
+    uint32_t w;
+    bool moved, turned, rec_set, set_v;            // new position; new orientation; new FP32 record; new velocities
+    d3 P, Ox, Oz, V, AV;
+    float4 rec, v32, w32;
+    double gone;                                   // a responding wall: how far any of its points went
+};
+__device__ __forceinline__ float4 wall_record(const SceneDev& S, uint32_t k1, int shape, const d3& Ox, const d3& Oz) {
+    const double lz = len(Oz), lx = len(Ox);
+    bool ok = lz > 0.0;
+    if (shape == SHAPE_PLATE || shape == SHAPE_HOLED) ok = ok && lx > 0.0 && fabs(dot(Ox, Oz)) <= 1e-9 * lx * lz;
+    const float nx = (float)(Oz.x / lz), ny = (float)(Oz.y / lz), nz = (float)(Oz.z / lz);
+    return ok ? make_float4(nx, ny, nz, frame_drift_across(S, k1, shape, nx, ny, nz)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+__device__ __forceinline__ bool walls_hold(const WallArgs& W) {
+    return list_spent(W.disp_in[0], W.disp_in[1], W.disp_in[2], W.skin, W.skin_w);
+}
+__device__ __forceinline__ WallStep wall_next(const WallArgs& W, uint32_t q) {
+    WallStep n;
+    const uint32_t w = n.w = W.glob[q];
+    n.moved = n.turned = n.rec_set = n.set_v = false;
+    n.P = ld(W.xA, w);
+    n.v32 = W.v32A[w];
+    n.w32 = W.w32A[w];
+    const SceneDev& S = W.scenes[W.scene_of[w]];
+    const ModelDev& M = W.models[W.model_of[w]];
+    if (walls_hold(W) || !S.active) return n;
     const double dt = S.dt;
-    const uint32_t k1 = __float_as_uint(disp_in[3]) + 1u;     // steps since the rebuild, after this one
-    d3 P = ld(xA, w);
+    const uint32_t k1 = __float_as_uint(W.disp_in[3]) + 1u;     // steps since the rebuild, after this one
+    n.moved = true;
     if (M.behavior == BEH_FIXED) {
-        float4 ws = wall32[w];
-        if (ws.w != 0.0f) {
-            ws.w = frame_drift_across(S, k1, M.shape, ws.x, ws.y, ws.z);
-            wall32[w] = ws;
+        n.rec = W.wall32[w];
+        if (n.rec.w != 0.0f) {
+            n.rec.w = frame_drift_across(S, k1, M.shape, n.rec.x, n.rec.y, n.rec.z);
+            n.rec_set = true;
         }
     } else if (M.behavior != BEH_ORBITAL) {
         // a mobile or constrained wall moved by its impulses this step (summed exactly by
         // k_wall_max/acc/fin, field and external force included), as the FP64 form's
         // respond_object: DOQuasiPlate.cpp:20-41 / DOConstrainedQuasiPlate.cpp:18-35
-        const d3 J = ld(imp, w), JA = ld(aimp, w);
-        d3 V = ld(v64, w), AV = ld(w64, w), Ox = ld(ox, w), Oz = ld(oz, w);
-        const d3 P0 = P;
+        const d3 J = ld(W.imp, w), JA = ld(W.aimp, w);
+        n.V = ld(W.v64, w);
+        n.AV = ld(W.w64, w);
+        n.Ox = ld(W.ox, w);
+        n.Oz = ld(W.oz, w);
+        const d3 P0 = n.P;
         d3 dw;
         if (M.behavior == BEH_CONSTRAINED) {
-            const d3 dv = smul(M.inv_sudo, smul(dot(J, Oz), dir(Oz)));
-            P = add(P, smul(dt, add(V, smul(0.5, dv))));
-            dw = muls(AV, dt);
-            V = add(V, dv);
+            const d3 dv = smul(M.inv_sudo, smul(dot(J, n.Oz), dir(n.Oz)));
+            n.P = add(n.P, smul(dt, add(n.V, smul(0.5, dv))));
+            dw = muls(n.AV, dt);
+            n.V = add(n.V, dv);
         } else {
             const d3 dv = smul(M.inv_sudo, J);
-            const d3 dav = mk(dot(JA, Ox) / M.ix, dot(JA, cross(Oz, Ox)) / M.iy, dot(JA, Oz) / M.iz);
-            P = add(P, smul(dt, add(V, smul(0.5, dv))));
-            dw = smul(dt, add(AV, smul(0.5, dav)));
-            V = add(V, dv);
-            AV = add(AV, dav);
+            const d3 dav = mk(dot(JA, n.Ox) / M.ix, dot(JA, cross(n.Oz, n.Ox)) / M.iy, dot(JA, n.Oz) / M.iz);
+            n.P = add(n.P, smul(dt, add(n.V, smul(0.5, dv))));
+            dw = smul(dt, add(n.AV, smul(0.5, dav)));
+            n.V = add(n.V, dv);
+            n.AV = add(n.AV, dav);
         }
         const Turn T = turn_of(dw);
-        Ox = rotate_by(Ox, T);
-        Oz = rotate_by(Oz, T);
-        st(ox, w, Ox, 0.0);
-        st(oz, w, Oz, 0.0);
-        st(v64, w, V, 0.0);
-        st(w64, w, AV, 0.0);
-        st(xB, w, P, 0.0);
-        v32B[w] = make_float4((float)V.x, (float)V.y, (float)V.z, 0.0f);
-        w32B[w] = make_float4((float)AV.x, (float)AV.y, (float)AV.z, 0.0f);
-        const double lz = len(Oz), lx = len(Ox);
-        bool ok = lz > 0.0;
-        if (M.shape == SHAPE_PLATE || M.shape == SHAPE_HOLED) ok = ok && lx > 0.0 && fabs(dot(Ox, Oz)) <= 1e-9 * lx * lz;
-        const float nx = (float)(Oz.x / lz), ny = (float)(Oz.y / lz), nz = (float)(Oz.z / lz);
-        wall32[w] = ok ? make_float4(nx, ny, nz, frame_drift_across(S, k1, M.shape, nx, ny, nz))
-                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        n.Ox = rotate_by(n.Ox, T);
+        n.Oz = rotate_by(n.Oz, T);
+        n.turned = n.rec_set = n.set_v = true;
+        n.v32 = make_float4((float)n.V.x, (float)n.V.y, (float)n.V.z, 0.0f);
+        n.w32 = make_float4((float)n.AV.x, (float)n.AV.y, (float)n.AV.z, 0.0f);
+        n.rec = wall_record(S, k1, M.shape, n.Ox, n.Oz);
         // how far any point of the wall went this step: its centre's travel and the turn of its
         // farthest point (k_wall_bound adds the largest to the walls' displacement bound)
         const double R = M.shape == SHAPE_INNER_CYL ? sqrt(M.a0 * M.a0 + 0.25 * M.a1 * M.a1)
                                                     : 0.5 * sqrt(M.a0 * M.a0 + M.a1 * M.a1 + M.a2 * M.a2);
-        const double d = len(sub(P, P0)) + len(dw) * R;
-        atomicMax(dyn_bits, __float_as_uint((float)(d * 1.0001) + 1e-30f));
-        return;
+        n.gone = len(sub(n.P, P0)) + len(dw) * R;
     } else {
-        const d3 V = ld(v64, w);
-        P = add(P, muls(V, dt));
+        n.P = add(n.P, muls(ld(W.v64, w), dt));
         // rotate_around(O, omega dt) with its cos/sin terms computed once per list (k_wall_rot)
-        const double4_32a R = wrot[q];
-        const d3 Ox = rotate_quat(ld(ox, w), R), Oz = rotate_quat(ld(oz, w), R);
-        st(ox, w, Ox, 0.0);
-        st(oz, w, Oz, 0.0);
-        const double lz = len(Oz), lx = len(Ox);
-        bool ok = lz > 0.0;
-        if (M.shape == SHAPE_PLATE || M.shape == SHAPE_HOLED) ok = ok && lx > 0.0 && fabs(dot(Ox, Oz)) <= 1e-9 * lx * lz;
-        const float nx = (float)(Oz.x / lz), ny = (float)(Oz.y / lz), nz = (float)(Oz.z / lz);
-        wall32[w] = ok ? make_float4(nx, ny, nz, frame_drift_across(S, k1, M.shape, nx, ny, nz))
-                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const double4_32a R = W.wrot[q];
+        n.Ox = rotate_quat(ld(W.ox, w), R);
+        n.Oz = rotate_quat(ld(W.oz, w), R);
+        n.turned = n.rec_set = true;
+        n.rec = wall_record(S, k1, M.shape, n.Ox, n.Oz);
     }
-    st(xB, w, P, 0.0);
-    v32B[w] = v32A[w];
-    w32B[w] = w32A[w];
+    return n;
 }
+__device__ __forceinline__ void wall_store(const WallArgs& W, const WallStep& n) {
+    if (n.moved) st(W.xB, n.w, n.P, 0.0);
+    else W.xB[n.w] = W.xA[n.w];
+    W.v32B[n.w] = n.v32;
+    W.w32B[n.w] = n.w32;
+    if (n.turned) {
+        st(W.ox, n.w, n.Ox, 0.0);
+        st(W.oz, n.w, n.Oz, 0.0);
+    }
+    if (n.rec_set) W.wall32[n.w] = n.rec;
+    if (n.set_v) {
+        st(W.v64, n.w, n.V, 0.0);
+        st(W.w64, n.w, n.AV, 0.0);
+        atomicMax(W.dyn_bits, __float_as_uint((float)(n.gone * 1.0001) + 1e-30f));
+    }
+}
+// The end of the step: the worklists emptied, the displacement bounds after it.
+__device__ __forceinline__ void step_end(const WallArgs& W) {
+    const float drel = W.disp_in[0], dabs = W.disp_in[1], dw = W.disp_in[2];
+    W.taken[0] = W.taken[1] = 0u;
+    W.nwork[0] = W.nwork[1] = 0u;                  // the worklists' counts (pair pass: wall pairs, then
+                                                   // sphere pairs and the split tick's spheres), empty
+                                                   // for the next step
+    if (walls_hold(W)) {
+        for (int k = 0; k < 4; ++k) W.disp_out[k] = W.disp_in[k];
+        *W.held += 1u;
+    } else {
+        // pos_eps: the FP64 rounding of a position update, which the speeds do not see
+        W.disp_out[0] = drel + W.dt_max * __uint_as_float(*W.vrel_bits) + W.pos_eps;
+        W.disp_out[1] = dabs + W.dt_max * __uint_as_float(*W.vmax_bits) + W.pos_eps;
+        W.disp_out[2] = dw + W.dt_max * __uint_as_float(*W.wall_speed_bits) + W.pos_eps;
+        W.disp_out[3] = __uint_as_float(__float_as_uint(W.disp_in[3]) + 1u);
+    }
+    *W.vmax_bits = 0u;
+    *W.vrel_bits = 0u;
+}
+__device__ __forceinline__ void walls_item(const WallArgs& W, uint32_t q) {
+    if (q == 0) step_end(W);
+    if (q < W.nglob) wall_store(W, wall_next(W, q));
+}
+// Between two steps this kernel is a serial chain (a wall's index, model and scene, its state, then
+// FP64 on one thread), 7 to 17 us when it ran after the step.  What it reads is the previous step's
+// and the list's, except a responding wall's impulses, and the kernels before that step's last one
+// have ended when it is launched; so it works its results out beside that last kernel and waits for
+// it (which may still read the walls) only to store them and to take the spheres' speeds.
 __global__ void k_walls(WallArgs W) {
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    WallStep n;
+    if (!W.dyn && q < W.nglob) n = wall_next(W, q);
     step_order();
-    walls_item(W, blockIdx.x * blockDim.x + threadIdx.x);
+    if (W.dyn && q < W.nglob) n = wall_next(W, q);
+    if (q == 0) step_end(W);
+    if (q < W.nglob) wall_store(W, n);
 }
 
 // After k_walls, when mobile or constrained walls move: the largest distance any point of such a
@@ -3551,6 +3552,7 @@ WallArgs MixedEngine::wargs(int c) {
     w.imp = d_imp_;
     w.aimp = d_aimp_;
     w.dyn_bits = d_red_ + 3;
+    w.dyn = dyn_walls_ ? 1 : 0;
     return w;
 }
 
