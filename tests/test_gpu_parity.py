@@ -438,3 +438,24 @@ def test_pair_kernel_candidates_per_block_bitexact(n_side, spacing, engine_lib, 
     ia, ib = e.interactions(), p.interactions()
     assert np.array_equal(ia["active"], ib["active"].astype(np.uint8))
     e.close()
+
+
+@pytest.mark.parametrize("n_side", [1, 2, 3, 8, 9, 10, 12, 13])
+def test_candidate_list_at_the_sorts_sizes(n_side, engine_lib, port_lib):
+    """Scenes whose cells and pair entries sort inside one block (to 2048 items), beside it and in
+    tiles, with rebuilds every step: candidate list, entries' order (the sums) and state bit for bit
+    against the oracle."""
+    from oracle import PortWorld
+    sc = scenes.lsd_box(n_side=n_side, steps=400, spacing=2.005e-3, vel_sigma=0.3, seed=n_side)
+    e = engine_lib.GpuEngine(sc, up_iact=1)
+    p = PortWorld(sc, up_iact=1)
+    for _ in range(4):
+        e.run(3)
+        p.run(3)
+        a, b = e.state(), p.state()
+        for k in ("position", "velocity", "angular_velocity", "impact", "angular_impact"):
+            np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+        ia = e.interactions()
+        f, s = p.candidates()
+        assert np.array_equal(ia["first"], f) and np.array_equal(ia["second"], s)
+    e.close()

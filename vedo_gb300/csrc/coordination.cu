@@ -363,12 +363,13 @@ static int coordination_device(uint32_t n, const uint32_t* model_of, const Model
     CN_CK(cudaMemsetAsync(nlt, 0, 8 * words, s));
     if (any) {
         CN_CK(cudaMemsetAsync(ce, 0, 4 * (size_t)ncell, s));
-        k_cn_keys<<<nblk(n), TPB, 0, s>>>(n, model_of, models, pos, g, ncell, key, id);
-        ++L;
         int bits = 1;
         while (bits < 32 && (ncell >> bits)) ++bits;
+        const bool alt = radix_passes_of(0, bits) & 1;
+        k_cn_keys<<<nblk(n), TPB, 0, s>>>(n, model_of, models, pos, g, ncell, alt ? key2 : key, alt ? id2 : id);
+        ++L;
         const uint64_t l0 = g_sort_scan_launches;
-        CN_CK(radix_sort_u32(key, id, key2, id2, n, 0, bits, scratch, s));
+        CN_CK(radix_sort_u32(key, id, key2, id2, n, 0, bits, scratch, s, alt));
         L += g_sort_scan_launches - l0;
         // the spheres' keys sort before the other shapes': the first ns entries
         if (ns) {

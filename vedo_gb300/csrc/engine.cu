@@ -1292,10 +1292,11 @@ int Engine::rebuild(bool from_records) {
     int bits = 1;
     while (bits < 64 && (sentinel >> bits)) ++bits;
     // 2. cell keys, stable sort (locals by cell in the comparator's order, ids ascending within a cell)
+    const bool kalt = radix_passes_of(0, bits) & 1;
     k_cellkey<<<blocks_for(n_), TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_pos_, xmin, ymin, zmin, zone, g,
-                                                   sentinel, d_key_, d_sid_);
+                                                   sentinel, kalt ? d_key_alt_ : d_key_, kalt ? d_sid_alt_ : d_sid_);
     ++own;
-    CK(radix_sort_u64(d_key_, d_sid_, d_key_alt_, d_sid_alt_, n_, 0, bits, scratch_, stream_));
+    CK(radix_sort_u64(d_key_, d_sid_, d_key_alt_, d_sid_alt_, n_, 0, bits, scratch_, stream_, kalt));
     // 3. cell ranges
     uint32_t np = 0;
     if (nloc) {
@@ -1376,11 +1377,13 @@ int Engine::rebuild(bool from_records) {
         CK(dalloc(&d_ck_, csr_cap_)); CK(dalloc(&d_ck_alt_, csr_cap_)); CK(dalloc(&d_cv_alt_, csr_cap_));
     }
     if (np) {
-        k_csr_keys<<<blocks_for(np), TPB, 0, stream_>>>(np, cur_.sm, d_ck_, cur_.csr_ent);
-        ++own;
         int obits = 1;
         while (obits < 32 && ((n_ - 1) >> obits)) ++obits;
-        CK(radix_sort_u32(d_ck_, cur_.csr_ent, d_ck_alt_, d_cv_alt_, m, 0, obits, scratch_, stream_));
+        const bool calt = radix_passes_of(0, obits) & 1;
+        k_csr_keys<<<blocks_for(np), TPB, 0, stream_>>>(np, cur_.sm, calt ? d_ck_alt_ : d_ck_,
+                                                        calt ? d_cv_alt_ : cur_.csr_ent);
+        ++own;
+        CK(radix_sort_u32(d_ck_, cur_.csr_ent, d_ck_alt_, d_cv_alt_, m, 0, obits, scratch_, stream_, calt));
     }
     k_csr_ptr<<<blocks_for((uint64_t)n_ + 1), TPB, 0, stream_>>>(n_, d_ck_, m, cur_.csr_ptr);
     ++own;

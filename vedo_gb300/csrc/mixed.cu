@@ -3737,12 +3737,13 @@ int MixedEngine::rebuild() {
     }
     MCK(cudaMemsetAsync(d_gs_, 0, 4 * cells, stream_));
     MCK(cudaMemsetAsync(d_ge_, 0, 4 * cells, stream_));
-    k_keys<<<nblk(n_), TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_scene_of_, d_scenes_, d_pos32_, cells,
-                                          d_key_, d_sid_);
-    ++own;
     int bits = 1;
     while (bits < 64 && (cells >> bits)) ++bits;
-    MCK(radix_sort_u64(d_key_, d_sid_, d_key_alt_, d_sid_alt_, n_, 0, bits, scratch_, stream_));
+    const bool kalt = radix_passes_of(0, bits) & 1;
+    k_keys<<<nblk(n_), TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_scene_of_, d_scenes_, d_pos32_, cells,
+                                          kalt ? d_key_alt_ : d_key_, kalt ? d_sid_alt_ : d_sid_);
+    ++own;
+    MCK(radix_sort_u64(d_key_, d_sid_, d_key_alt_, d_sid_alt_, n_, 0, bits, scratch_, stream_, kalt));
     if (nloc_) {
         k_cells<<<nblk(nloc_), TPB, 0, stream_>>>(nloc_, d_key_, d_gs_, d_ge_);
         ++own;
@@ -3808,10 +3809,12 @@ int MixedEngine::rebuild() {
             MCK(mal(&d_wval_alt_, wcap_));
         }
         nwall_ent_ = nw;
-        k_wall_fill<<<nblk(n_), TPB, 0, stream_>>>(n_, L.ptr, L.ent, d_cnt_, d_gidx_, d_wkey_, d_wval_);
         int wb = 1;
         while (wb < 32 && (((uint32_t)glob_.size() - 1) >> wb)) ++wb;
-        MCK(radix_sort_u32(d_wkey_, d_wval_, d_wkey_alt_, d_wval_alt_, nw, 0, wb, scratch_, stream_));
+        const bool walt = radix_passes_of(0, wb) & 1;
+        k_wall_fill<<<nblk(n_), TPB, 0, stream_>>>(n_, L.ptr, L.ent, d_cnt_, d_gidx_, walt ? d_wkey_alt_ : d_wkey_,
+                                                   walt ? d_wval_alt_ : d_wval_);
+        MCK(radix_sort_u32(d_wkey_, d_wval_, d_wkey_alt_, d_wval_alt_, nw, 0, wb, scratch_, stream_, walt));
         k_wall_ptr<<<nblk(glob_.size() + 1), TPB, 0, stream_>>>((uint32_t)glob_.size(), d_wkey_, nw, d_wptr_);
         own += 3;
         if (6ull * ne > wimp_cap_) {
