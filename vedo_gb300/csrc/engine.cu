@@ -66,6 +66,17 @@ __host__ __device__ inline uint64_t grid_key(const CellGrid& g, const uint64_t c
     return (c[0] * g.dim[1] + c[1]) * g.dim[2] + c[2];
 }
 __device__ inline void grid_cell(const CellGrid& g, uint64_t key, uint64_t c[3]) {
+    if (key <= 0xffffffffull) {        // (nearly always) 32-bit divisions
+        const uint32_t k = (uint32_t)key, lo = (uint32_t)(g.mode == 1 ? g.dim[2] : g.mode == 2 ? g.dim[1] : g.dim[2]),
+                       mid = (uint32_t)(g.mode == 1 ? g.dim[0] : g.mode == 2 ? g.dim[0] : g.dim[1]);
+        if (g.dim[0] <= 0xffffffffull && g.dim[1] <= 0xffffffffull && g.dim[2] <= 0xffffffffull) {
+            const uint32_t q = k / lo, first = q / mid, second = q % mid, third = k % lo;
+            if (g.mode == 1) { c[1] = first; c[0] = second; c[2] = third; }
+            else if (g.mode == 2) { c[2] = first; c[0] = second; c[1] = third; }
+            else { c[0] = first; c[1] = second; c[2] = third; }
+            return;
+        }
+    }
     if (g.mode == 1) {
         c[2] = key % g.dim[2]; key /= g.dim[2]; c[0] = key % g.dim[0]; c[1] = key / g.dim[0];
     } else if (g.mode == 2) {
@@ -451,42 +462,47 @@ __global__ void __launch_bounds__(TPB) k_detect_active(uint32_t np, const uint2*
 
 // ------------------------------------------------------------------------------------
 // broad phase (NBSConsultant::Reset, NBSConsultant.cpp:85-316)
+// (A few blocks per SM, each reduced to one set of atomics: eight same-address 64-bit atomics a warp
+// took 29 us for 150,000 objects.)
 __global__ void __launch_bounds__(TPB) k_safe(uint32_t n, const uint32_t* __restrict__ model_of,
                                               const ModelDev* __restrict__ models, const double4_32a* __restrict__ pos,
                                               const double4_32a* __restrict__ vel, double sf, double dtu, double glen,
                                               double* __restrict__ safe, unsigned long long* __restrict__ red) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long mn[3] = {~0ull, ~0ull, ~0ull}, mx[3] = {0, 0, 0}, vm = 0, last = 0;
-    if (i < n) {
+    __shared__ unsigned long long sh[8][TPB / 32];
+    unsigned long long v[8] = {~0ull, 0, ~0ull, 0, ~0ull, 0, 0, 0};    // min, max per axis; speed; last local object + 1
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const ModelDev& m = models[model_of[i]];
         const double vl = len(ld(vel, i));
         safe[i] = sf * (2.0 * m.range + dtu * vl + 0.5 * dtu * dtu * glen);   // :127-129
-        if (m.scope == SCOPE_LOCAL) {                                          // :131-141
-            const double4_32a p = pos[i];
-            mn[0] = mx[0] = ord_of(p.x);
-            mn[1] = mx[1] = ord_of(p.y);
-            mn[2] = mx[2] = ord_of(p.z);
-            vm = ord_of(vl);
-            last = (unsigned long long)i + 1;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+        if (m.scope != SCOPE_LOCAL) continue;                                  // :131-141
+        const double4_32a p = pos[i];
+        const unsigned long long o[3] = {ord_of(p.x), ord_of(p.y), ord_of(p.z)};
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            mn[q] = min(mn[q], __shfl_xor_sync(0xffffffffu, mn[q], o));
-            mx[q] = max(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
+            v[2 * q] = min(v[2 * q], o[q]);
+            v[2 * q + 1] = max(v[2 * q + 1], o[q]);
         }
-        vm = max(vm, __shfl_xor_sync(0xffffffffu, vm, o));
-        last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
+        v[6] = max(v[6], ord_of(vl));
+        v[7] = max(v[7], (unsigned long long)i + 1);
     }
-    if ((threadIdx.x & 31) == 0) {
-        for (int q = 0; q < 3; ++q) {
-            atomicMin(&red[2 * q], mn[q]);
-            atomicMax(&red[2 * q + 1], mx[q]);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const bool least = q < 6 && !(q & 1);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long x = __shfl_xor_sync(0xffffffffu, v[q], o);
+            v[q] = least ? min(v[q], x) : max(v[q], x);
         }
-        atomicMax(&red[6], vm);
-        atomicMax(&red[7], last);
+        if ((threadIdx.x & 31) == 0) sh[q][threadIdx.x >> 5] = v[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        const int q = threadIdx.x;
+        const bool least = q < 6 && !(q & 1);
+        unsigned long long x = sh[q][0];
+        for (int w = 1; w < TPB / 32; ++w) x = least ? min(x, sh[q][w]) : max(x, sh[q][w]);
+        if (least) atomicMin(&red[q], x);
+        else atomicMax(&red[q], x);
     }
 }
 
@@ -532,10 +548,20 @@ __global__ void __launch_bounds__(TPB) k_cell_flags(uint32_t nloc, const uint64_
     flag[p] = (p == 0 || key[p] != key[p - 1]) ? 1u : 0u;
 }
 
+// One sphere's part of the distance beyond which a pair of spheres is certainly no candidate: its safe
+// length, rounded up, and the rounding of its FP32 position (prefilter.cuh's dist32 bound).
+__device__ __forceinline__ float pair_limit(const float4& q, double safe) {
+    return (float)safe * (1.0f + 16.0f * PF_ARITH_EPS) + PF_POS_EPS * 1.0001f * l1(q);
+}
 __global__ void __launch_bounds__(TPB) k_cell_fill(uint32_t nloc, const uint64_t* __restrict__ key,
                                                    const uint32_t* __restrict__ flag_excl,
                                                    uint64_t* __restrict__ cell_key, uint32_t* __restrict__ cell_start,
-                                                   uint32_t* __restrict__ cellof, const uint32_t* __restrict__ ncells) {
+                                                   uint32_t* __restrict__ cellof, const uint32_t* __restrict__ ncells,
+                                                   uint32_t* __restrict__ grid,
+                                                   const uint32_t* __restrict__ sid, const uint32_t* __restrict__ model_of,
+                                                   const ModelDev* __restrict__ models,
+                                                   const float4* __restrict__ pos32, const double* __restrict__ safe,
+                                                   float4* __restrict__ rec) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nloc) return;
     const bool head = (p == 0 || key[p] != key[p - 1]);
@@ -544,8 +570,14 @@ __global__ void __launch_bounds__(TPB) k_cell_fill(uint32_t nloc, const uint64_t
     if (head) {
         cell_key[c] = key[p];
         cell_start[c] = p;
+        if (grid) grid[key[p]] = c;                              // the dense map of a small grid
     }
     if (p == nloc - 1) cell_start[*ncells] = nloc;
+    // what the candidate test reads of an object, in cell order: its FP32 position, and its safe length
+    // with its share of the test's error allowance (other shapes: no pair with them is settled by it)
+    const uint32_t i = sid[p];
+    const float4 q = pos32[i];
+    rec[p] = make_float4(q.x, q.y, q.z, models[model_of[i]].shape == SHAPE_SPHERE ? pair_limit(q, safe[i]) : __int_as_float(0x7f800000));
 }
 
 // Candidate test of BuildIactTab (NBSConsultant.cpp:318-345): DOMap::CalDistance <= safe_i +
@@ -602,8 +634,10 @@ __device__ __forceinline__ bool candidate(const ModelDev& mi, const ModelDev& mj
 // One thread per (slot, object) task, slot-major so that a warp works on one slot.  Tasks
 // are numbered in the reference's traversal order: cell by cell (ix, iy, iz lexicographic),
 // within a cell by slot, within a slot by the object's position in the cell (ascending id).
+// The count pass leaves which of a task's objects are candidates in a word (tasks of up to 32, nearly
+// all), so that the fill pass evaluates no distance again.
 template <bool FILL>
-__global__ void __launch_bounds__(TPB) k_pairs(uint32_t nloc, const uint32_t* __restrict__ sid,
+__global__ void __launch_bounds__(TPB, 3) k_pairs(uint32_t nloc, const uint32_t* __restrict__ sid,
                                                const uint64_t* __restrict__ cell_key,
                                                const uint32_t* __restrict__ cell_start,
                                                const uint32_t* __restrict__ ncells_p, const uint32_t* __restrict__ cellof,
@@ -614,8 +648,11 @@ __global__ void __launch_bounds__(TPB) k_pairs(uint32_t nloc, const uint32_t* __
                                                const double4_32a* __restrict__ pos, const double4_32a* __restrict__ ox,
                                                const double4_32a* __restrict__ oz, const float4* __restrict__ pos32,
                                                const float4* __restrict__ wall32, const double* __restrict__ safe,
-                                               CellGrid g, Periodic pbv,
-                                               uint32_t* __restrict__ task, uint32_t* __restrict__ first,
+                                               const float4* __restrict__ rec,
+                                               CellGrid g, Periodic pbv, uint32_t nm,
+                                               const uint8_t* __restrict__ refused,
+                                               uint32_t* __restrict__ task, uint32_t* __restrict__ picked,
+                                               uint32_t* __restrict__ first,
                                                uint32_t* __restrict__ second, int* __restrict__ err) {
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (uint64_t)nloc * NSLOT) return;
@@ -626,6 +663,14 @@ __global__ void __launch_bounds__(TPB) k_pairs(uint32_t nloc, const uint32_t* __
     grid_cell(g, cell_key[c], cc);
     const uint32_t cs = cell_start[c], csize = cell_start[c + 1] - cs;
     const uint64_t tid = (uint64_t)cs * NSLOT + (uint64_t)s * csize + (P - cs);
+    // the fill pass knows each task's count from the scanned offsets (the next task's offset, or
+    // the total after the last one): it stops at its last candidate and skips empty tasks
+    const uint32_t off = FILL ? task[tid] : 0u;
+    uint32_t want = 0xffffffffu;
+    if (FILL) {
+        want = ((uint64_t)tid + 1 < (uint64_t)nloc * NSLOT ? task[tid + 1] : ncells_p[1]) - off;
+        if (want == 0u) return;
+    }
     // NBS: only cells inside the loops are primary (:186-190); Leap visits every zone of its map
     if (!g.leap && (cc[0] >= g.ncel[0] || cc[1] >= g.ncel[1] || cc[2] >= g.ncel[2])) {
         if (!FILL) task[tid] = 0;
@@ -694,19 +739,37 @@ __global__ void __launch_bounds__(TPB) k_pairs(uint32_t nloc, const uint32_t* __
         }
     }
     const uint32_t i = sid[P];
-    const ModelDev& mi = models[model_of[i]];
+    uint32_t cnt = 0;
+    if (FILL && jn <= 32u) {
+        for (uint32_t m = picked[t]; m; m &= m - 1u) {
+            const uint32_t j = js[__ffs((int)m) - 1];
+            first[off + cnt] = i < j ? i : j;
+            second[off + cnt] = i < j ? j : i;
+            ++cnt;
+        }
+        return;
+    }
+    const uint32_t mdi = model_of[i];
+    const ModelDev& mi = models[mdi];
     const double si = safe[i];
     const float si32 = (float)si;
     const int gi = mi.group;
-    uint32_t cnt = 0;
-    const uint32_t off = FILL ? task[tid] : 0u;
-    // the fill pass knows each task's count from the scanned offsets (the next task's offset, or
-    // the total after the last one): it stops at its last candidate and skips empty tasks
-    uint32_t want = 0xffffffffu;
-    if (FILL) want = ((uint64_t)tid + 1 < (uint64_t)nloc * NSLOT ? task[tid + 1] : ncells_p[1]) - off;
+    uint32_t mask = 0u;
+    // spheres of a cell against a sphere: the records in cell order settle nearly all that are no
+    // candidates from one contiguous load and a squared distance
+    const bool quick = s != slot_global && mi.shape == SHAPE_SPHERE && !(g.leap && pbv.on);
+    const uint32_t b0 = quick && jn ? (uint32_t)(js - sid) : 0u;
+    const float4 pi32 = pos32[i];
+    const float mine = pair_limit(pi32, si);
     for (uint32_t q = 0; q < jn && cnt < want; ++q) {
+        if (quick) {
+            const float4 r = rec[b0 + q];
+            const float dx = r.x - pi32.x, dy = r.y - pi32.y, dz = r.z - pi32.z, lim = mine + r.w;
+            if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) > lim * lim * (1.0f + 16.0f * PF_ARITH_EPS)) continue;
+        }
         const uint32_t j = js[q];
-        const ModelDev& mj = models[model_of[j]];
+        const uint32_t mdj = model_of[j];
+        const ModelDev& mj = models[mdj];
         if (group_iact[gi * G + mj.group] < 0) continue;
         const double sj = safe[j];
         if (!candidate(mi, mj, i, j, si, sj, si32, (float)sj, pos, ox, oz, pos32, wall32, err,
@@ -714,16 +777,17 @@ __global__ void __launch_bounds__(TPB) k_pairs(uint32_t nloc, const uint32_t* __
         if (FILL) {
             first[off + cnt] = i < j ? i : j;
             second[off + cnt] = i < j ? j : i;
+        } else {
+            if (q < 32u) mask |= 1u << q;
+            // no interaction of an object with itself (Assembler.cpp:27-30): the Leap consultant lists such
+            // pairs when a periodic axis is one zone wide, and the reference then drops them, leaving its
+            // pair table and interactions misaligned; here the list is refused
+            if (i == j || refused[i < j ? mdi * nm + mdj : mdj * nm + mdi]) atomicOr(err, ERR_UNSUPPORTED_PAIR);
         }
         ++cnt;
     }
+    if (!FILL) picked[t] = mask;
     if (!FILL) task[tid] = cnt;
-}
-
-__global__ void __launch_bounds__(TPB) k_grid_fill(const uint32_t* __restrict__ ncells_p,
-                                                   const uint64_t* __restrict__ cell_key, uint32_t* __restrict__ grid) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < *ncells_p) grid[cell_key[c]] = c;
 }
 
 __global__ void __launch_bounds__(TPB) k_refresh32(uint32_t n, const uint32_t* __restrict__ model_of,
@@ -737,126 +801,123 @@ __global__ void __launch_bounds__(TPB) k_refresh32(uint32_t n, const uint32_t* _
     write32(i, models[model_of[i]].shape, ld(pos, i), ld(ox, i), ld(oz, i), origin, pos32, wall32);
 }
 
-// Assembler::CreateInteraction orientation and model selection (Assembler.cpp:15-87)
-__global__ void __launch_bounds__(TPB) k_setup(uint32_t np, const uint32_t* __restrict__ first,
+// What a new pair needs, in one pass over the list: its orientation and model (Assembler::
+// CreateInteraction, Assembler.cpp:15-87), its two per-object entries to be sorted, and its history.
+// REC: from the IactRecordTab read with the scene (IactRecordTab::GetImpactStatus, IactRecordTab.cpp:20-25;
+// records sorted by (first << 32 | second)).  Else carried: the status of the same (first, second) pair of
+// the old list when that pair is active at the present positions (RebuildIactRecordTab + Initiate,
+// NBSConsultant.cpp:376-395, SimMediator.cpp:690-707), otherwise a default-constructed ImpactStatus.  Only a
+// new pair that is active needs the old list, so the narrow phase runs on the pairs near contact here and
+// not on every pair of the old list first, and in full warps like k_pair's (150,000-sphere drum: set-up,
+// that pass, carry and entries took 211 us, 269 in one pass with a lane each, 187 like this).
+constexpr uint32_t SETUP_MAX = 4;     // most rounds of pairs a block takes
+struct HistorySource {
+    const uint64_t* rkey;              // records
+    uint32_t nrec;
+    const double4_32a* hist;           // records, or the old list
+    const double* v0;
+    const uint8_t* flags;
+    const uint32_t *ptr, *ent, *first, *second;     // the old list
+};
+template <bool REC>
+__global__ void __launch_bounds__(TPB) k_setup(uint32_t np, uint32_t per, const uint32_t* __restrict__ first,
                                                const uint32_t* __restrict__ second,
                                                const uint32_t* __restrict__ model_of,
                                                const ModelDev* __restrict__ models,
                                                const PairParam* __restrict__ params, uint32_t nm,
-                                               uint2* __restrict__ sm, uint32_t* __restrict__ param,
-                                               int* __restrict__ err) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= np) return;
-    const uint32_t a = first[k], b = second[k];
-    const uint32_t ma = model_of[a], mb = model_of[b];
-    const ModelDev& A = models[ma];
-    const ModelDev& B = models[mb];
-    uint32_t sl = a, ms = b;
-    // no interaction of an object with itself (Assembler.cpp:27-30): the Leap consultant lists such
-    // pairs when a periodic axis is one zone wide, and the reference then drops them, leaving its
-    // pair table and interactions misaligned; here the list is refused
-    bool bad = a == b || (B.density < 0.0 || A.density < 0.0) || (B.density == 0.0 && A.density == 0.0);
-    if (A.shape > B.shape) { sl = b; ms = a; }
-    else if (A.shape < B.shape) { sl = a; ms = b; }
-    else if (A.density == 0.0) { sl = b; ms = a; }
-    else if (B.density == 0.0) { sl = a; ms = b; }
-    const uint32_t pi = model_of[sl] * nm + model_of[ms];
-    if (bad || params[pi].cd == 0) {
-        atomicOr(err, ERR_UNSUPPORTED_PAIR);
-        sm[k] = make_uint2(a, b);
-        param[k] = 0;
-        return;
-    }
-    sm[k] = make_uint2(sl, ms);
-    param[k] = pi;
-}
-
-// History carry: a new pair takes the status of the same (first, second) pair of the old
-// list when that pair was active (RebuildIactRecordTab + Initiate, NBSConsultant.cpp:376-395,
-// SimMediator.cpp:690-707); otherwise a default-constructed ImpactStatus.
-__global__ void __launch_bounds__(TPB) k_history_old(uint32_t np, const uint32_t* __restrict__ first,
-                                                     const uint32_t* __restrict__ second,
-                                                     const uint2* __restrict__ sm, const uint32_t* __restrict__ param,
-                                                     const PairParam* __restrict__ params,
-                                                     const float* __restrict__ reach,
-                                                     const float4* __restrict__ pos32,
-                                                     const float4* __restrict__ wall32,
-                                                     const uint32_t* __restrict__ o_ptr,
-                                                     const uint32_t* __restrict__ o_ent,
-                                                     const uint32_t* __restrict__ o_first,
-                                                     const uint32_t* __restrict__ o_second,
-                                                     const uint8_t* __restrict__ o_flags,
-                                                     const double4_32a* __restrict__ o_hist,
-                                                     const double* __restrict__ o_v0, double4_32a* __restrict__ hist,
-                                                     double* __restrict__ v0, uint8_t* __restrict__ flags,
-                                                     Periodic pb) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= np) return;
-    const uint32_t a = first[k], b = second[k];
-    uint8_t f = ST_DEFAULT;
-    double4_32a h = make_double4_32a(0.0, 0.0, 0.0, 0.0);
-    double vv = 0.0;
-    const uint2 p = sm[k];
-    const uint32_t pi = param[k];
-    // a pair certainly apart now was not active at this position in the old list either
-    const bool maybe = !certainly_apart(params[pi].cd, pos32[p.x], pos32[p.y], wall32[p.y], reach[pi],
-                                        pb.on ? pb.range32 : nullptr);
-    const uint32_t e1 = maybe ? o_ptr[a + 1] : 0u;
-    for (uint32_t e = maybe ? o_ptr[a] : 0u; e < e1; ++e) {
-        const uint32_t ko = o_ent[e] >> 1;
-        if (o_first[ko] == a && o_second[ko] == b) {
-            const uint8_t of = o_flags[ko];
-            if (of & PF_ACTIVE) {
-                f = of & (PF_STATUS | PF_NONZERO);
-                if (of & PF_NONZERO) {
-                    h = o_hist[ko];
-                    vv = o_v0[ko];
-                }
+                                               const uint8_t* __restrict__ refused,
+                                               const double4_32a* __restrict__ geom, const double4_32a* __restrict__ hole,
+                                               const float* __restrict__ reach, const double4_32a* __restrict__ pos,
+                                               const double4_32a* __restrict__ ox, const double4_32a* __restrict__ oz,
+                                               const float4* __restrict__ pos32, const float4* __restrict__ wall32,
+                                               Periodic pb, HistorySource src, uint2* __restrict__ sm,
+                                               uint32_t* __restrict__ param, uint32_t* __restrict__ ckey,
+                                               uint32_t* __restrict__ cval, double4_32a* __restrict__ hist,
+                                               double* __restrict__ v0, uint8_t* __restrict__ flags) {
+    __shared__ uint32_t list[SETUP_MAX * TPB];
+    __shared__ uint32_t count;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    for (uint32_t r = 0; r < per; ++r) {
+        const uint32_t k = (blockIdx.x * per + r) * TPB + threadIdx.x;
+        bool near = false;
+        if (k < np) {
+            const uint32_t a = first[k], b = second[k];
+            const uint32_t ma = model_of[a], mb = model_of[b];
+            const ModelDev& A = models[ma];
+            const ModelDev& B = models[mb];
+            uint2 p = make_uint2(a, b);
+            if (A.shape > B.shape) p = make_uint2(b, a);
+            else if (A.shape == B.shape && A.density == 0.0) p = make_uint2(b, a);
+            uint32_t pi = p.x == a ? ma * nm + mb : mb * nm + ma;
+            if (a == b || refused[ma * nm + mb]) {            // (the list is refused)
+                p = make_uint2(a, b);
+                pi = 0;
             }
+            sm[k] = p;
+            param[k] = pi;
+            reinterpret_cast<uint2*>(ckey)[k] = p;
+            reinterpret_cast<uint2*>(cval)[k] = make_uint2(2 * k, 2 * k + 1);
+            uint8_t f = ST_DEFAULT;
+            double4_32a h = make_double4_32a(0.0, 0.0, 0.0, 0.0);
+            double vv = 0.0;
+            if (REC) {
+                const uint64_t key = ((uint64_t)a << 32) | b;
+                uint32_t lo = 0, hi = src.nrec;
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (src.rkey[mid] < key) lo = mid + 1; else hi = mid;
+                }
+                if (lo < src.nrec && src.rkey[lo] == key) {
+                    h = src.hist[lo];
+                    vv = src.v0[lo];
+                    f = src.flags[lo];
+                }
+            } else {
+                near = params[pi].cd != 0 && !certainly_apart(params[pi].cd, pos32[p.x], pos32[p.y], wall32[p.y],
+                                                              reach[pi], pb.on ? pb.range32 : nullptr);
+            }
+            hist[k] = h;
+            v0[k] = vv;
+            flags[k] = f;
+        }
+        if (REC) continue;
+        const unsigned m = __ballot_sync(0xffffffffu, near);
+        uint32_t at = 0;
+        if (lane == 0 && m) at = atomicAdd(&count, (uint32_t)__popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (near) list[at + __popc(m & ((1u << lane) - 1u))] = k;
+    }
+    if (REC) return;
+    __syncthreads();
+    const uint32_t nw = count;
+    for (uint32_t q = threadIdx.x; q < nw; q += TPB) {         // the FP64 narrow phase in full warps
+        const uint32_t k = list[q], pi = param[k];
+        const uint2 p = sm[k];
+        const double4_32a gg = geom[pi];
+        PairGeom g{gg.x, gg.y, gg.z, gg.w, 0.0, 0.0, 0.0};
+        if (params[pi].cd == CD_SHP) {
+            const double4_32a hh = hole[pi];
+            g.hr = hh.x; g.hxo = hh.y; g.hyo = hh.z;
+        }
+        double depth;
+        d3 n, point;
+        detect_pair(params[pi].cd, g, ld(pos, p.x), ld(pos, p.y), ox, oz, p.y, pb, depth, n, point);
+        if (!(depth > 0.0)) continue;
+        const uint32_t a = first[k], b = second[k], e1 = src.ptr[a + 1];
+        for (uint32_t e = src.ptr[a]; e < e1; ++e) {
+            const uint32_t ko = src.ent[e] >> 1;
+            if (src.first[ko] != a || src.second[ko] != b) continue;
+            const uint8_t of = src.flags[ko];
+            if (of & PF_NONZERO) {
+                hist[k] = src.hist[ko];
+                v0[k] = src.v0[ko];
+            }
+            flags[k] = of & (PF_STATUS | PF_NONZERO);
             break;
         }
     }
-    hist[k] = h;
-    v0[k] = vv;
-    flags[k] = f;
-}
-
-// History from the IactRecordTab read with the scene (IactRecordTab::GetImpactStatus,
-// IactRecordTab.cpp:20-25); records are sorted by (first << 32 | second).
-__global__ void __launch_bounds__(TPB) k_history_rec(uint32_t np, const uint32_t* __restrict__ first,
-                                                     const uint32_t* __restrict__ second,
-                                                     const uint64_t* __restrict__ rkey, uint32_t nrec,
-                                                     const double4_32a* __restrict__ rhist, const double* __restrict__ rv0,
-                                                     const uint8_t* __restrict__ rflags, double4_32a* __restrict__ hist,
-                                                     double* __restrict__ v0, uint8_t* __restrict__ flags) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= np) return;
-    const uint64_t key = ((uint64_t)first[k] << 32) | second[k];
-    uint32_t lo = 0, hi = nrec;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (rkey[mid] < key) lo = mid + 1; else hi = mid;
-    }
-    if (lo < nrec && rkey[lo] == key) {
-        hist[k] = rhist[lo];
-        v0[k] = rv0[lo];
-        flags[k] = rflags[lo];
-    } else {
-        hist[k] = make_double4_32a(0.0, 0.0, 0.0, 0.0);
-        v0[k] = 0.0;
-        flags[k] = ST_DEFAULT;
-    }
-}
-
-__global__ void __launch_bounds__(TPB) k_csr_keys(uint32_t np, const uint2* __restrict__ sm, uint32_t* __restrict__ key,
-                                                  uint32_t* __restrict__ val) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= np) return;
-    const uint2 p = sm[k];
-    key[2 * k] = p.x;
-    val[2 * k] = 2 * k;
-    key[2 * k + 1] = p.y;
-    val[2 * k + 1] = 2 * k + 1;
 }
 
 __global__ void __launch_bounds__(TPB) k_csr_ptr(uint32_t n, const uint32_t* __restrict__ key, uint32_t m,
@@ -919,7 +980,7 @@ Engine::~Engine() {
     if (stream_) cudaStreamSynchronize(stream_);
     free_list(cur_);
     free_list(old_);
-    void* ptrs[] = {d_models_, d_params_, d_geom_, d_group_iact_, d_model_of_, d_err_, d_pos_, d_vel_, d_av_, d_ox_,
+    void* ptrs[] = {d_models_, d_params_, d_geom_, d_group_iact_, d_model_of_, d_refused_, d_picked_, d_bp_, d_pos_, d_vel_, d_av_, d_ox_,
                     d_oz_, d_imp_, d_aimp_, d_global_, d_safe_, d_red_, d_key_, d_key_alt_, d_cell_key_, d_sid_,
                     d_sid_alt_, d_cell_start_, d_cellof_, d_flag_, d_task_, d_total_, d_ck_, d_cv_, d_ck_alt_,
                     d_cv_alt_, d_cnt_, d_rec_key_, d_rec_hist_, d_rec_v0_, d_rec_flags_, d_obs_, d_stage_,
@@ -975,8 +1036,20 @@ int Engine::init(const HScene& scene, const vedo_engine_opts& opts) {
     CK(cudaMemcpy(d_group_iact_, tab_.group_iact.data(), sizeof(int) * G * G, cudaMemcpyHostToDevice));
     CK(dalloc(&d_model_of_, n_));
     CK(cudaMemcpy(d_model_of_, host_.model_of.data(), sizeof(uint32_t) * n_, cudaMemcpyHostToDevice));
-    CK(dalloc(&d_err_, 1));
-    CK(cudaMemset(d_err_, 0, sizeof(int)));
+    // pairs of models the Assembler makes no interaction of (Assembler.cpp:27-87), by the models of the
+    // lower and the higher object
+    std::vector<uint8_t> refused((size_t)nm_ * nm_);
+    for (uint32_t a = 0; a < nm_; ++a)
+        for (uint32_t b = 0; b < nm_; ++b) {
+            const ModelDev &A = tab_.models[a], &B = tab_.models[b];
+            bool swap = false;                                 // the higher object is the slave
+            if (A.shape > B.shape) swap = true;
+            else if (A.shape == B.shape) swap = A.density == 0.0;
+            refused[(size_t)a * nm_ + b] = A.density < 0.0 || B.density < 0.0 || (A.density == 0.0 && B.density == 0.0) ||
+                                           tab_.params[swap ? (size_t)b * nm_ + a : (size_t)a * nm_ + b].cd == 0;
+        }
+    CK(dalloc(&d_refused_, refused.size()));
+    CK(cudaMemcpy(d_refused_, refused.data(), refused.size(), cudaMemcpyHostToDevice));
     // objects
     std::vector<double4_32a> tmp;
     double4_32a** dst[] = {&d_pos_, &d_vel_, &d_av_, &d_ox_, &d_oz_, &d_imp_, &d_aimp_};
@@ -1029,6 +1102,7 @@ int Engine::init(const HScene& scene, const vedo_engine_opts& opts) {
     // broad-phase scratch
     CK(dalloc(&d_safe_, n_)); CK(dalloc(&d_red_, 8)); CK(dalloc(&d_key_, n_)); CK(dalloc(&d_key_alt_, n_));
     CK(dalloc(&d_cell_key_, n_)); CK(dalloc(&d_sid_, n_)); CK(dalloc(&d_sid_alt_, n_));
+    CK(dalloc(&d_bp_, n_));
     CK(dalloc(&d_cell_start_, (size_t)n_ + 1)); CK(dalloc(&d_cellof_, n_)); CK(dalloc(&d_flag_, n_));
     CK(dalloc(&d_total_, 4));
     CK(dalloc(&d_obs_, (size_t)(blocks_for(n_) + 2) * 16 + 64));
@@ -1221,13 +1295,6 @@ int Engine::status_row_now() {
 int Engine::rebuild(bool from_records) {
     const uint64_t l0 = g_sort_scan_launches;
     uint64_t own = 0;
-    // IsActive() of the current interactions at the current positions
-    if (!from_records && cur_.np) {
-        k_detect_active<<<blocks_for(cur_.np), TPB, 0, stream_>>>(cur_.np, cur_.sm, cur_.param, d_params_, d_geom_,
-                                                                  d_hole_, d_reach_, d_pos_, d_ox_, d_oz_, d_pos32_,
-                                                                  d_wall32_, cur_.flags, tab_.pbc);
-        ++own;
-    }
     std::swap(cur_, old_);
     // 1. safe lengths and bounds (:120-146)
     const double dtu = (double)opts_.up_iact * dt_;
@@ -1235,7 +1302,7 @@ int Engine::rebuild(bool from_records) {
     unsigned long long red0[8] = {ord_of(DBL_MAX), ord_of(DBL_MIN), ord_of(DBL_MAX), ord_of(DBL_MIN),
                                   ord_of(DBL_MAX), ord_of(DBL_MIN), ord_of(0.0), 0ull};
     CK(cudaMemcpyAsync(d_red_, red0, sizeof(red0), cudaMemcpyHostToDevice, stream_));
-    k_safe<<<blocks_for(n_), TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_pos_, d_vel_, sf_, dtu, glen, d_safe_,
+    k_safe<<<std::min(blocks_for(n_), 608u), TPB, 0, stream_>>>(n_, d_model_of_, d_models_, d_pos_, d_vel_, sf_, dtu, glen, d_safe_,
                                                 d_red_);
     ++own;
     unsigned long long red[8];
@@ -1299,20 +1366,8 @@ int Engine::rebuild(bool from_records) {
     CK(radix_sort_u64(d_key_, d_sid_, d_key_alt_, d_sid_alt_, n_, 0, bits, scratch_, stream_, kalt));
     // 3. cell ranges
     uint32_t np = 0;
+    int herr = 0;
     if (nloc) {
-        k_cell_flags<<<blocks_for(nloc), TPB, 0, stream_>>>(nloc, d_key_, d_flag_);
-        CK(exclusive_scan_u32(d_flag_, d_flag_, nloc, d_total_, scratch_, stream_));
-        k_cell_fill<<<blocks_for(nloc), TPB, 0, stream_>>>(nloc, d_key_, d_flag_, d_cell_key_, d_cell_start_,
-                                                           d_cellof_, d_total_);
-        own += 2;
-        // 4. count pass over (object, slot) tasks, scan, fill pass
-        const uint64_t ntask = (uint64_t)nloc * NSLOT;
-        if (ntask + 1 > task_cap_) {
-            if (d_task_) cudaFree(d_task_);
-            task_cap_ = (uint32_t)(ntask + 1);
-            CK(dalloc(&d_task_, task_cap_));
-        }
-        CK(cudaMemsetAsync(d_err_, 0, sizeof(int), stream_));
         // dense cell map when the grid is small compared with the object count
         uint32_t* grid = nullptr;
         const uint64_t gcells = sentinel;
@@ -1324,49 +1379,51 @@ int Engine::rebuild(bool from_records) {
                 CK(dalloc(&d_grid_, grid_cap_));
             }
             CK(cudaMemsetAsync(d_grid_, 0xff, sizeof(uint32_t) * gcells, stream_));
-            k_grid_fill<<<blocks_for(nloc), TPB, 0, stream_>>>(d_total_, d_cell_key_, d_grid_);
-            ++own;
             grid = d_grid_;
         }
+        k_cell_flags<<<blocks_for(nloc), TPB, 0, stream_>>>(nloc, d_key_, d_flag_);
+        CK(exclusive_scan_u32(d_flag_, d_flag_, nloc, d_total_, scratch_, stream_));
+        k_cell_fill<<<blocks_for(nloc), TPB, 0, stream_>>>(nloc, d_key_, d_flag_, d_cell_key_, d_cell_start_,
+                                                           d_cellof_, d_total_, grid, d_sid_, d_model_of_, d_models_, d_pos32_,
+                                                           d_safe_, d_bp_);
+        own += 2;
+        // 4. count pass over (object, slot) tasks, scan, fill pass
+        const uint64_t ntask = (uint64_t)nloc * NSLOT;
+        if (ntask + 1 > task_cap_) {
+            if (d_task_) cudaFree(d_task_);
+            if (d_picked_) cudaFree(d_picked_);
+            d_task_ = d_picked_ = nullptr;
+            task_cap_ = (uint32_t)(ntask + 1);
+            CK(dalloc(&d_task_, task_cap_));
+            CK(dalloc(&d_picked_, task_cap_));
+        }
+        int* err = reinterpret_cast<int*>(d_total_ + 2);
+        CK(cudaMemsetAsync(err, 0, sizeof(int), stream_));
         k_pairs<false><<<blocks_for(ntask), TPB, 0, stream_>>>(
             nloc, d_sid_, d_cell_key_, d_cell_start_, d_total_, d_cellof_, grid, gcells, d_global_,
             (uint32_t)global_ids_.size(), d_model_of_, d_models_, d_group_iact_, tab_.ngroups, d_pos_, d_ox_, d_oz_,
-            d_pos32_, d_wall32_, d_safe_, g, tab_.pbc, d_task_, nullptr, nullptr, d_err_);
+            d_pos32_, d_wall32_, d_safe_, d_bp_, g, tab_.pbc, nm_, d_refused_, d_task_, d_picked_, nullptr, nullptr, err);
         ++own;
         CK(exclusive_scan_u32(d_task_, d_task_, (uint32_t)ntask, d_total_ + 1, scratch_, stream_));
-        CK(cudaMemcpyAsync(&np, d_total_ + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_));
+        uint32_t got[2];
+        CK(cudaMemcpyAsync(got, d_total_ + 1, sizeof(got), cudaMemcpyDeviceToHost, stream_));
         CK(cudaStreamSynchronize(stream_));
+        np = got[0];
+        herr = (int)got[1];
         int rc = ensure_list(cur_, np);
         if (rc != VEDO_OK) return rc;
         k_pairs<true><<<blocks_for(ntask), TPB, 0, stream_>>>(
             nloc, d_sid_, d_cell_key_, d_cell_start_, d_total_, d_cellof_, grid, gcells, d_global_,
             (uint32_t)global_ids_.size(), d_model_of_, d_models_, d_group_iact_, tab_.ngroups, d_pos_, d_ox_, d_oz_,
-            d_pos32_, d_wall32_, d_safe_, g, tab_.pbc, d_task_, cur_.first, cur_.second, d_err_);
+            d_pos32_, d_wall32_, d_safe_, d_bp_, g, tab_.pbc, nm_, d_refused_, d_task_, d_picked_, cur_.first, cur_.second, err);
         ++own;
     } else {
         int rc = ensure_list(cur_, 0);
         if (rc != VEDO_OK) return rc;
     }
     cur_.np = np;
-    // 5. interactions: orientation and model selection
-    if (np) {
-        k_setup<<<blocks_for(np), TPB, 0, stream_>>>(np, cur_.first, cur_.second, d_model_of_, d_models_, d_params_,
-                                                     nm_, cur_.sm, cur_.param, d_err_);
-        ++own;
-        // 6. history
-        if (from_records) {
-            k_history_rec<<<blocks_for(np), TPB, 0, stream_>>>(np, cur_.first, cur_.second, d_rec_key_, nrec_,
-                                                               d_rec_hist_, d_rec_v0_, d_rec_flags_, cur_.hist,
-                                                               cur_.v0, cur_.flags);
-        } else {
-            k_history_old<<<blocks_for(np), TPB, 0, stream_>>>(np, cur_.first, cur_.second, cur_.sm, cur_.param,
-                                                               d_params_, d_reach_, d_pos32_, d_wall32_, old_.csr_ptr,
-                                                               old_.csr_ent, old_.first, old_.second, old_.flags,
-                                                               old_.hist, old_.v0, cur_.hist, cur_.v0, cur_.flags, tab_.pbc);
-        }
-        ++own;
-    }
-    // 7. per-object contact entries in ascending pair index (stable radix sort by object)
+    // 5. interactions: orientation, model, history; 6. per-object contact entries in ascending pair
+    // index (stable radix sort by object)
     const uint32_t m = 2 * np;
     if (m > csr_cap_) {
         for (uint32_t** p : {&d_ck_, &d_ck_alt_, &d_cv_alt_}) {
@@ -1380,16 +1437,21 @@ int Engine::rebuild(bool from_records) {
         int obits = 1;
         while (obits < 32 && ((n_ - 1) >> obits)) ++obits;
         const bool calt = radix_passes_of(0, obits) & 1;
-        k_csr_keys<<<blocks_for(np), TPB, 0, stream_>>>(np, cur_.sm, calt ? d_ck_alt_ : d_ck_,
-                                                        calt ? d_cv_alt_ : cur_.csr_ent);
+        const HistorySource src = from_records ? HistorySource{d_rec_key_, nrec_, d_rec_hist_, d_rec_v0_, d_rec_flags_,
+                                                               nullptr, nullptr, nullptr, nullptr}
+                                               : HistorySource{nullptr, 0, old_.hist, old_.v0, old_.flags, old_.csr_ptr,
+                                                               old_.csr_ent, old_.first, old_.second};
+        auto k = from_records ? k_setup<true> : k_setup<false>;
+        const uint32_t per = np >= SETUP_MAX * TPB * 304u ? SETUP_MAX : 1u;    // a block for every SM first
+        k<<<blocks_for(np, (int)(per * TPB)), TPB, 0, stream_>>>(np, per, cur_.first, cur_.second, d_model_of_, d_models_, d_params_, nm_,
+                                               d_refused_, d_geom_, d_hole_, d_reach_, d_pos_, d_ox_, d_oz_, d_pos32_,
+                                               d_wall32_, tab_.pbc, src, cur_.sm, cur_.param, calt ? d_ck_alt_ : d_ck_,
+                                               calt ? d_cv_alt_ : cur_.csr_ent, cur_.hist, cur_.v0, cur_.flags);
         ++own;
         CK(radix_sort_u32(d_ck_, cur_.csr_ent, d_ck_alt_, d_cv_alt_, m, 0, obits, scratch_, stream_, calt));
     }
     k_csr_ptr<<<blocks_for((uint64_t)n_ + 1), TPB, 0, stream_>>>(n_, d_ck_, m, cur_.csr_ptr);
     ++own;
-    int herr = 0;
-    CK(cudaMemcpyAsync(&herr, d_err_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
-    CK(cudaStreamSynchronize(stream_));
     CK(cudaGetLastError());
     launches_ += own + (g_sort_scan_launches - l0);
     if (herr & ERR_BAD_SHAPE_PAIR)

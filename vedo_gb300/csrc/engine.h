@@ -106,7 +106,7 @@ private:
     double4_32a* d_hole_ = nullptr;     // per (slave model, master model): hole radius, offsets (CD_SHP)
     int* d_group_iact_ = nullptr;
     uint32_t* d_model_of_ = nullptr;
-    int* d_err_ = nullptr;
+    uint8_t* d_refused_ = nullptr;      // per (lower, higher object's model): no interaction is made of the pair
     // device: objects
     double4_32a *d_pos_ = nullptr, *d_vel_ = nullptr, *d_av_ = nullptr, *d_ox_ = nullptr, *d_oz_ = nullptr;
     double4_32a *d_imp_ = nullptr, *d_aimp_ = nullptr;
@@ -121,8 +121,9 @@ private:
     unsigned long long* d_red_ = nullptr;
     uint64_t *d_key_ = nullptr, *d_key_alt_ = nullptr, *d_cell_key_ = nullptr;
     uint32_t *d_sid_ = nullptr, *d_sid_alt_ = nullptr, *d_cell_start_ = nullptr, *d_cellof_ = nullptr;
-    uint32_t *d_flag_ = nullptr, *d_task_ = nullptr, *d_total_ = nullptr;
+    uint32_t *d_flag_ = nullptr, *d_task_ = nullptr, *d_picked_ = nullptr, *d_total_ = nullptr;
     uint32_t task_cap_ = 0;
+    float4* d_bp_ = nullptr;             // local objects in cell order: FP32 position, pair_limit
     uint32_t *d_ck_ = nullptr, *d_cv_ = nullptr, *d_ck_alt_ = nullptr, *d_cv_alt_ = nullptr;
     uint32_t csr_cap_ = 0;
     uint32_t* d_cnt_ = nullptr;
