@@ -183,7 +183,7 @@ template <int PER>
 __global__ void __launch_bounds__(TPB) k_pair(uint32_t np, const uint2* __restrict__ sm,
                                               const uint32_t* __restrict__ param, const PairParam* __restrict__ params,
                                               const double4_32a* __restrict__ geom,
-                                              const double4_32a* __restrict__ hole, const float* __restrict__ reach,
+                                              const double4_32a* __restrict__ hole, const float2* __restrict__ brief,
                                               const double4_32a* __restrict__ pos, const double4_32a* __restrict__ vel,
                                               const double4_32a* __restrict__ av, const double4_32a* __restrict__ ox,
                                               const double4_32a* __restrict__ oz, const float4* __restrict__ pos32,
@@ -210,11 +210,10 @@ __global__ void __launch_bounds__(TPB) k_pair(uint32_t np, const uint2* __restri
         const uint32_t k = base + r * TPB;
         bool near = false;
         if (k < np) {
-            const int cd = params[pi[r]].cd, is = params[pi[r]].is;
-            const bool bondable =
-                (is == IS_BSDBF || is == IS_BTSDBF || is == IS_BSDB2F) && params[pi[r]].c[4] != 0.0;
-            if (!bondable && certainly_apart(cd, pos32[p[r].x], pos32[p[r].y], wall32[p[r].y], reach[pi[r]],
-                                             pb.on ? pb.range32 : nullptr)) {
+            const float2 br = brief[pi[r]];
+            const int cd = __float_as_int(br.y);
+            if (cd && certainly_apart(cd, pos32[p[r].x], pos32[p[r].y], wall32[p[r].y], br.x,
+                                      pb.on ? pb.range32 : nullptr)) {
                 const uint8_t f0 = flags[k];
                 if (f0 & PF_NONZERO) {
                     hist[k] = make_double4_32a(0.0, 0.0, 0.0, 0.0);
@@ -649,7 +648,7 @@ __global__ void __launch_bounds__(TPB, 3) k_pairs(uint32_t nloc, const uint32_t*
                                                const double4_32a* __restrict__ oz, const float4* __restrict__ pos32,
                                                const float4* __restrict__ wall32, const double* __restrict__ safe,
                                                const float4* __restrict__ rec,
-                                               CellGrid g, Periodic pbv, uint32_t nm,
+                                               CellGrid g, Periodic pbv, uint32_t nm, int all_interact,
                                                const uint8_t* __restrict__ refused,
                                                uint32_t* __restrict__ task, uint32_t* __restrict__ picked,
                                                uint32_t* __restrict__ first,
@@ -760,12 +759,26 @@ __global__ void __launch_bounds__(TPB, 3) k_pairs(uint32_t nloc, const uint32_t*
     const bool quick = s != slot_global && mi.shape == SHAPE_SPHERE && !(g.leap && pbv.on);
     const uint32_t b0 = quick && jn ? (uint32_t)(js - sid) : 0u;
     const float4 pi32 = pos32[i];
-    const float mine = pair_limit(pi32, si);
+    const float mine = pair_limit(pi32, si), slack = 2.1f * PF_POS_EPS * l1(pi32);
     for (uint32_t q = 0; q < jn && cnt < want; ++q) {
         if (quick) {
             const float4 r = rec[b0 + q];
             const float dx = r.x - pi32.x, dy = r.y - pi32.y, dz = r.z - pi32.z, lim = mine + r.w;
-            if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) > lim * lim * (1.0f + 16.0f * PF_ARITH_EPS)) continue;
+            const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            if (d2 > lim * lim * (1.0f + 16.0f * PF_ARITH_EPS)) continue;
+            // certainly within: the limits less twice their allowances (an infinite one: not settled here)
+            const float in = lim * (1.0f - 64.0f * PF_ARITH_EPS) - slack - 2.1f * PF_POS_EPS * l1(r);
+            if (all_interact && lim < 3e38f && in > 0.0f && d2 < in * in * (1.0f - 16.0f * PF_ARITH_EPS)) {
+                if (FILL) {
+                    const uint32_t j = js[q];
+                    first[off + cnt] = i < j ? i : j;
+                    second[off + cnt] = i < j ? j : i;
+                } else if (q < 32u) {
+                    mask |= 1u << q;
+                }
+                ++cnt;
+                continue;
+            }
         }
         const uint32_t j = js[q];
         const uint32_t mdj = model_of[j];
@@ -980,7 +993,7 @@ Engine::~Engine() {
     if (stream_) cudaStreamSynchronize(stream_);
     free_list(cur_);
     free_list(old_);
-    void* ptrs[] = {d_models_, d_params_, d_geom_, d_group_iact_, d_model_of_, d_refused_, d_picked_, d_bp_, d_pos_, d_vel_, d_av_, d_ox_,
+    void* ptrs[] = {d_models_, d_params_, d_geom_, d_group_iact_, d_model_of_, d_refused_, d_picked_, d_bp_, d_brief_, d_pos_, d_vel_, d_av_, d_ox_,
                     d_oz_, d_imp_, d_aimp_, d_global_, d_safe_, d_red_, d_key_, d_key_alt_, d_cell_key_, d_sid_,
                     d_sid_alt_, d_cell_start_, d_cellof_, d_flag_, d_task_, d_total_, d_ck_, d_cv_, d_ck_alt_,
                     d_cv_alt_, d_cnt_, d_rec_key_, d_rec_hist_, d_rec_v0_, d_rec_flags_, d_obs_, d_stage_,
@@ -1048,6 +1061,14 @@ int Engine::init(const HScene& scene, const vedo_engine_opts& opts) {
             refused[(size_t)a * nm_ + b] = A.density < 0.0 || B.density < 0.0 || (A.density == 0.0 && B.density == 0.0) ||
                                            tab_.params[swap ? (size_t)b * nm_ + a : (size_t)a * nm_ + b].cd == 0;
         }
+    // whether every two sphere models interact: the candidate test then needs no look at the models
+    all_interact_ = 1;
+    for (uint32_t a = 0; a < nm_; ++a)
+        for (uint32_t b = 0; b < nm_; ++b)
+            if (tab_.models[a].shape == SHAPE_SPHERE && tab_.models[b].shape == SHAPE_SPHERE &&
+                (refused[(size_t)a * nm_ + b] ||
+                 tab_.group_iact[(size_t)tab_.models[a].group * tab_.ngroups + tab_.models[b].group] < 0))
+                all_interact_ = 0;
     CK(dalloc(&d_refused_, refused.size()));
     CK(cudaMemcpy(d_refused_, refused.data(), refused.size(), cudaMemcpyHostToDevice));
     // objects
@@ -1089,6 +1110,19 @@ int Engine::init(const HScene& scene, const vedo_engine_opts& opts) {
             if (tab_.params[q].cd == CD_SIC) reach[q] = (float)(gq[0] - gq[1]) * (1.0f - 1e-6f);
             else reach[q] = (float)r * (1.0f + 1e-6f);
         }
+        // what k_pair's prefilter reads of a pair's models: reach and detector, no detector (the pair is
+        // always evaluated) where the law may bond
+        std::vector<float2> brief(reach.size());
+        for (size_t q = 0; q < reach.size(); ++q) {
+            const PairParam& P = tab_.params[q];
+            const bool bondable = (P.is == IS_BSDBF || P.is == IS_BTSDBF || P.is == IS_BSDB2F) && P.c[4] != 0.0;
+            const int cd = bondable ? 0 : P.cd;
+            float w;
+            memcpy(&w, &cd, 4);
+            brief[q] = make_float2(reach[q], w);
+        }
+        CK(dalloc(&d_brief_, brief.size()));
+        CK(cudaMemcpy(d_brief_, brief.data(), sizeof(float2) * brief.size(), cudaMemcpyHostToDevice));
         CK(dalloc(&d_reach_, reach.size()));
         CK(cudaMemcpy(d_reach_, reach.data(), sizeof(float) * reach.size(), cudaMemcpyHostToDevice));
         k_refresh32<<<blocks_for(n_), TPB>>>(n_, d_model_of_, d_models_, d_pos_, d_ox_, d_oz_,
@@ -1402,7 +1436,7 @@ int Engine::rebuild(bool from_records) {
         k_pairs<false><<<blocks_for(ntask), TPB, 0, stream_>>>(
             nloc, d_sid_, d_cell_key_, d_cell_start_, d_total_, d_cellof_, grid, gcells, d_global_,
             (uint32_t)global_ids_.size(), d_model_of_, d_models_, d_group_iact_, tab_.ngroups, d_pos_, d_ox_, d_oz_,
-            d_pos32_, d_wall32_, d_safe_, d_bp_, g, tab_.pbc, nm_, d_refused_, d_task_, d_picked_, nullptr, nullptr, err);
+            d_pos32_, d_wall32_, d_safe_, d_bp_, g, tab_.pbc, nm_, all_interact_, d_refused_, d_task_, d_picked_, nullptr, nullptr, err);
         ++own;
         CK(exclusive_scan_u32(d_task_, d_task_, (uint32_t)ntask, d_total_ + 1, scratch_, stream_));
         uint32_t got[2];
@@ -1415,7 +1449,7 @@ int Engine::rebuild(bool from_records) {
         k_pairs<true><<<blocks_for(ntask), TPB, 0, stream_>>>(
             nloc, d_sid_, d_cell_key_, d_cell_start_, d_total_, d_cellof_, grid, gcells, d_global_,
             (uint32_t)global_ids_.size(), d_model_of_, d_models_, d_group_iact_, tab_.ngroups, d_pos_, d_ox_, d_oz_,
-            d_pos32_, d_wall32_, d_safe_, d_bp_, g, tab_.pbc, nm_, d_refused_, d_task_, d_picked_, cur_.first, cur_.second, err);
+            d_pos32_, d_wall32_, d_safe_, d_bp_, g, tab_.pbc, nm_, all_interact_, d_refused_, d_task_, d_picked_, cur_.first, cur_.second, err);
         ++own;
     } else {
         int rc = ensure_list(cur_, 0);
@@ -1477,7 +1511,7 @@ int Engine::step_once(bool write_impulses) {
         const uint32_t per = cur_.np >= 8u * TPB * 304u ? 8u : cur_.np >= 4u * TPB * 152u ? 4u : 2u;
         auto k = per == 8u ? k_pair<8> : per == 4u ? k_pair<4> : k_pair<2>;
         k<<<blocks_for(cur_.np, (int)(per * TPB)), TPB, 0, stream_>>>(
-            cur_.np, cur_.sm, cur_.param, d_params_, d_geom_, d_hole_, d_reach_, d_pos_, d_vel_, d_av_, d_ox_, d_oz_,
+            cur_.np, cur_.sm, cur_.param, d_params_, d_geom_, d_hole_, d_brief_, d_pos_, d_vel_, d_av_, d_ox_, d_oz_,
             d_pos32_, d_wall32_, cur_.hist, cur_.v0, cur_.flags, cur_.out, dt, backup_pending_ ? 1 : 0, tab_.pbc,
             d_touched_);
         ++launches_;

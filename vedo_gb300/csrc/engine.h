@@ -143,6 +143,8 @@ private:
     double leap_rmax_ = 0.0;
     float4* d_wall32_ = nullptr;
     float* d_reach_ = nullptr;
+    float2* d_brief_ = nullptr;     // per (slave model, master model): reach, detector (k_pair's prefilter)
+    int all_interact_ = 0;          // every two sphere models interact
     double origin_[3] = {0, 0, 0};
     // dense cell -> cell-index map of the broad phase when the grid is small enough
     uint32_t* d_grid_ = nullptr;

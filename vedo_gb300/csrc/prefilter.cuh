@@ -76,8 +76,13 @@ __device__ __forceinline__ float dist32_periodic(const float4& a, const float4& 
 __device__ __forceinline__ bool certainly_apart(int cd, const float4& s, const float4& m, const float4& wall,
                                                 float reach, const float* periodic = nullptr) {
     float e, d;
-    if (cd == 1) {
-        d = periodic ? dist32_periodic(s, m, periodic, e) : dist32(s, m, e);
+    if (cd == 1 && !periodic) {
+        // the squared distance against the reach with the allowances on its side: no square root
+        const float dx = m.x - s.x, dy = m.y - s.y, dz = m.z - s.z;
+        const float lim = reach * (1.0f + 4.0f * PF_ARITH_EPS) + PF_POS_EPS * (l1(s) + l1(m));
+        return dx * dx + dy * dy + dz * dz > lim * lim * (1.0f + 8.0f * PF_ARITH_EPS);
+    } else if (cd == 1) {
+        d = dist32_periodic(s, m, periodic, e);
     } else if (cd == 2 || cd == 4) {
         if (wall.w == 0.0f) return false;
         d = plane_dist32(s, m, wall, e);
