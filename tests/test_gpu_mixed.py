@@ -444,3 +444,19 @@ def test_pair_worklists_handed_out_in_chunks(n, block, engine_lib):
             assert np.array_equal(sa[f], sb[f]), f
     a.close()
     b.close()
+
+
+def test_tick_of_a_large_dense_packing(engine_lib):
+    """The full tick with a thread per sphere (large lists of ten entries a sphere and more) against the
+    pair pass: identical bits."""
+    sc = scenes.dense_pack(n=200003, steps=1000)
+    a = engine_lib.GpuEngine(sc, precision=1)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True)
+    for k in (1, 11):
+        a.run(k)
+        b.run(k)
+        sa, sb = a.state(), b.state()
+        for f in ("position", "velocity", "angular_velocity", "impact", "angular_impact"):
+            assert np.array_equal(sa[f], sb[f]), f
+    a.close()
+    b.close()

@@ -1116,6 +1116,21 @@ __global__ void __launch_bounds__(TPB, 2) k_tick(TickArgs a, int lanes) {
     reduce_vmax(a, vmax_local);
 }
 
+// The full tick with one thread per sphere, for large dense packings (launch_tick's rule): there the
+// shared slots above overflow and cost the gathers their cache, and every lane has pairs anyway.
+template <int LAW, bool XS>
+__global__ void __launch_bounds__(TPB) k_tick_each(TickArgs a) {
+    step_order();
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    float2 vmax_local = make_float2(0.0f, 0.0f);
+    if (held_step(a)) {                          // the same value for every thread of the launch
+        hold_state(a, t);
+    } else if (t < a.n) {
+        vmax_local = tick_sphere<LAW, XS>(a, t);
+    }
+    reduce_vmax(a, vmax_local);
+}
+
 // The full tick of the split tick: a grid sized to the resident threads strides over the
 // spheres the light kernel deferred (none in a held step).
 template <int LAW, bool XS>
@@ -1392,16 +1407,16 @@ __device__ __forceinline__ void pairs_from(const TickArgs& a, uint32_t first, ui
 // others ended (700,000 spheres in 48 hoppers: 445 us a step with the two kernels side by side, 355 one
 // after the other, 320 like this; 1,000,000 packed spheres 508 to 480).  A list of at most a pair a thread is taken as it lies: every warp
 // asking at once costs about 1 ns each on the one counter (60,000-sphere hopper: 47 us a step so, 57
-// asking).  Longer ones go in about eight chunks a warp, the first of the blocks that surely start at
+// asking), and one of at most two where few wall pairs take room from it (60,000 spheres in a box: 32
+// against 40).  Longer ones go in about eight chunks a warp, the first of the blocks that surely start at
 // once fixed, the next one asked for before the present one is worked on.
 template <int LAW, bool XS, int KIND>
 __device__ __forceinline__ void pairs_taken(const TickArgs& a) {
-    const uint32_t nw = min(a.nwork[0], a.pcap), count = KIND == 1 ? nw : min(a.nwork[-1], a.pcap - nw);
+    const uint32_t nw = min(a.nwork[0], a.pcap), nww = min(a.nwork[-1], a.pcap - nw), count = KIND == 1 ? nw : nww;
     const uint32_t threads = gridDim.x * blockDim.x;
     auto item = [&](uint32_t q) { pair_item<LAW, XS, KIND>(a, a.pwork[KIND == 1 ? q : a.pcap - 1u - q]); };
-    if (count <= threads) {
-        const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-        if (q < count) item(q);
+    if (count <= threads || (KIND == 1 && count <= 2u * threads && nww < count / 16u)) {
+        for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += threads) item(q);
         return;
     }
     const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5, given = gridDim.x / 2u * wpb;
@@ -2909,7 +2924,7 @@ private:
     }
     int rebuild();
     void launch_step(bool write_imp);
-    cudaError_t launch_tick(bool dep, void (*k)(TickArgs, int), const TickArgs& a);
+    cudaError_t launch_tick(bool dep, void (*k)(TickArgs, int), void (*each)(TickArgs), const TickArgs& a);
     cudaError_t launch_err_ = cudaSuccess;   // the first failed launch of the step kernels
     int step_chunk(uint32_t chunk, bool imp_last, float* use_after);
     int autotune(uint32_t max_steps, uint32_t* taken);
@@ -3886,17 +3901,24 @@ static cudaError_t step_launch(bool dep, void (*k)(P...), unsigned grid, unsigne
 }
 
 // The full tick's launch.  Threads per sphere: 8 or 4 while that keeps every sphere of the scene resident
-// at once (512 threads an SM at the tick's registers), 2 up to two rounds of that, then 1.  us per step
-// at 1 / 2 / 4 / 8 (GB300): 8,000-sphere box 37 / 29 / 26 / 24; 10,000 loose spheres 12 / 12 / 12 / 14;
-// 20,000 packed 71 / 55 / 64 / 69; 40,000-sphere drum 39 / 34 / 36 / 44; 60,000-sphere hopper 74 / 60 /
-// 73 / 102; 200,000 packed 224 / 257 / 350 / 485.  A scene that leaves SMs without a block takes smaller
-// blocks than tick_block, down to 64 threads (2,000-sphere hopper, 256 to 64: 35 to 27).
-cudaError_t MixedEngine::launch_tick(bool dep, void (*k)(TickArgs, int), const TickArgs& a) {
+// at once (512 threads an SM at the tick's registers), 2 to five eighths of that many spheres, then 1, in
+// blocks of at most 128.  us per step at 1 / 2 / 4 / 8 (GB300): 8,000-sphere box 37 / 29 / 26 / 24; 10,000
+// loose spheres 12 / 12 / 12 / 14; 20,000 packed 71 / 55 / 64 / 69; 40,000-sphere drum 39 / 34 / 36 / 44;
+// 60,000 in the box 32 / 37, loose 13 / 15, packed 74 / 88, in a hopper 63 / 58; 200,000 packed 218 / 257.
+// A scene that leaves SMs without a block takes smaller blocks than tick_block, down to 64 threads
+// (2,000-sphere hopper, 256 to 64: 35 to 27).  From 2.5 times the resident spheres on, lists of ten
+// entries a sphere and more take the kernel with a thread per sphere (packings of 100,000 / 300,000: 121
+// against its 136, 284 against its 256).
+cudaError_t MixedEngine::launch_tick(bool dep, void (*k)(TickArgs, int), void (*each)(TickArgs), const TickArgs& a) {
     const uint64_t room = (uint64_t)sms_ * 512u;
-    int lanes = n_ <= room ? 1 : 0;
+    if (2ull * n_ > 5u * room && nl_[nlc_].ne >= 10ull * n_)
+        return step_launch(dep, each, (unsigned)((n_ + tpb_ - 1) / tpb_), (unsigned)tpb_, stream_, a);
+    int lanes = 8ull * n_ <= 5u * room ? 1 : 0;
     while (lanes >= 1 && lanes < 3 && ((uint64_t)n_ << (lanes + 1)) <= room) ++lanes;
     unsigned block = (unsigned)tpb_;
-    while (block >= 128u && block % 64u == 0u && ((uint64_t)n_ << lanes) < (uint64_t)sms_ * block) block /= 2u;
+    while (block >= 128u && block % 64u == 0u &&
+           (((uint64_t)n_ << lanes) < (uint64_t)sms_ * block || (lanes == 0 && block > 128u)))
+        block /= 2u;
     const unsigned spheres = block >> lanes;
     const size_t bytes = (size_t)tick_slots(spheres) * (2 * sizeof(float4) + sizeof(uint2));
     if (bytes > 48 * 1024) {
@@ -3968,7 +3990,8 @@ void MixedEngine::launch_step(bool write_imp) {
         note(step_launch(dep, xs_stored_ ? k_tick_work<L, true> : k_tick_work<L, false>, nb_full,            \
                          (unsigned)tpb_, stream_, a));                                                       \
     else                                                                                                    \
-        note(launch_tick(dep, xs_stored_ ? k_tick<L, true> : k_tick<L, false>, a))
+        note(launch_tick(dep, xs_stored_ ? k_tick<L, true> : k_tick<L, false>,                              \
+                         xs_stored_ ? k_tick_each<L, true> : k_tick_each<L, false>, a))
     switch (law_) {
     case IS_BSDBF: VEDO_TICK(IS_BSDBF); break;
     case IS_BTSDBF: VEDO_TICK(IS_BTSDBF); break;
