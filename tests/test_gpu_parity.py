@@ -422,9 +422,9 @@ def test_system_status_csv_matches_reference(case, engine_lib, tmp_path):
 
 @pytest.mark.parametrize("n_side,spacing", [(8, 2.4e-3), (12, 2.005e-3), (24, 2.005e-3), (34, 2.005e-3), (45, 2.005e-3)])
 def test_pair_kernel_candidates_per_block_bitexact(n_side, spacing, engine_lib, port_lib):
-    """The pair kernel at each of its block sizes (512, 1024 and 2048 candidates, remainders
-    included) and on a list of which it keeps nothing: 30 steps of colliding linear-law spheres with
-    rebuilds every 7, bit for bit against the oracle."""
+    """The pair kernel on lists of less than a tile to several tiles a block, remainders included, and
+    on one of which it keeps nothing: 30 steps of colliding linear-law spheres with rebuilds every 7,
+    bit for bit against the oracle."""
     from oracle import PortWorld
     sc = scenes.lsd_box(n_side=n_side, steps=400, spacing=spacing, vel_sigma=0.3, box_width=n_side * spacing + 1e-3,
                         box_height=n_side * spacing + 5e-3)

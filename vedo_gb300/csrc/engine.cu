@@ -172,15 +172,19 @@ __device__ __forceinline__ void pair_exact(uint32_t k, const uint2* __restrict__
 }
 
 // CalculateImpact.  The FP64 pipe issues a warp instruction in 16 cycles however few of its lanes are
-// active, and most candidate pairs are apart, so a block first settles its PER * 256 candidates with
-// the FP32 prefilter (a pair certainly apart that carries no normal bond gets ImpactStatus::Clean and
-// no impulse), compacting the others in shared memory, and then evaluates those in full warps: narrow
-// phase at the current positions, impact solver, status update, each pair's operations those of a
-// pass over the list (their order does not matter, every pair writes its own records).  While one
-// block waits for its gathers the FP64 pipe works on another's.  PER: the more candidates a block
-// compacts, the fuller its last warp, but a short list has to spread over the SMs (step_once).
-template <int PER>
-__global__ void __launch_bounds__(TPB) k_pair(uint32_t np, const uint2* __restrict__ sm,
+// active, and most candidate pairs are apart, so the pairs that need it are evaluated in full warps: the
+// blocks resident at once take the list's tiles of 512 candidates in turn, settle them with the FP32
+// prefilter (a pair certainly apart that carries no normal bond gets ImpactStatus::Clean and no impulse)
+// and put the others aside in shared memory until there is one for every thread; then narrow phase at
+// the present positions, impact solver and status update, each pair's operations those of a pass over
+// the list (their order does not matter, every pair writes its own records).  While one block waits for
+// its gathers the FP64 pipe works on another's.  With tiles of fixed size per block, evaluated alone, a
+// list of a few waves lost up to half in the last rounds (us per step, 60,000-sphere hopper, 58,000
+// packed, 150,000-sphere drum: 349, 517, 245; 255, 458, 249 like this; 284, 488, 313 with a prefilter
+// kernel and a worklist in memory).  Three blocks an SM at 80 registers and a few spills, against two at
+// 112: 255 to 263, 458 to 472, 249 to 267.
+constexpr int PAIR_TILE = 2;      // candidates a thread settles per tile
+__global__ void __launch_bounds__(TPB, 3) k_pair(uint32_t np, const uint2* __restrict__ sm,
                                               const uint32_t* __restrict__ param, const PairParam* __restrict__ params,
                                               const double4_32a* __restrict__ geom,
                                               const double4_32a* __restrict__ hole, const float2* __restrict__ brief,
@@ -191,50 +195,66 @@ __global__ void __launch_bounds__(TPB) k_pair(uint32_t np, const uint2* __restri
                                               double* __restrict__ v0, uint8_t* __restrict__ flags,
                                               double* __restrict__ out, double dt, int backup, Periodic pb,
                                               uint8_t* __restrict__ touched) {
-    __shared__ uint32_t list[PER * TPB];
+    __shared__ uint32_t list[(PAIR_TILE + 1) * TPB];          // fewer than TPB, and a tile's
     __shared__ uint32_t count;
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) count = 0;
     __syncthreads();
-    const uint32_t base = blockIdx.x * (uint32_t)(PER * TPB) + threadIdx.x;
-    uint2 p[PER];
-    uint32_t pi[PER];
+    const uint32_t tiles = (np + PAIR_TILE * TPB - 1u) / (PAIR_TILE * TPB);
+    uint32_t t = blockIdx.x, n = 0;                            // n: the pairs put aside (the same in every thread)
+    for (;;) {
+        while (n < TPB && t < tiles) {
+            const uint32_t base = t * (uint32_t)(PAIR_TILE * TPB) + threadIdx.x;
+            t += gridDim.x;
+            uint2 p[PAIR_TILE];
+            uint32_t pi[PAIR_TILE];
 #pragma unroll
-    for (int r = 0; r < PER; ++r) {                            // (the candidates' loads overlap)
-        const uint32_t k = base + r * TPB;
-        p[r] = k < np ? sm[k] : make_uint2(0u, 0u);
-        pi[r] = k < np ? param[k] : 0u;
-    }
-#pragma unroll
-    for (int r = 0; r < PER; ++r) {
-        const uint32_t k = base + r * TPB;
-        bool near = false;
-        if (k < np) {
-            const float2 br = brief[pi[r]];
-            const int cd = __float_as_int(br.y);
-            if (cd && certainly_apart(cd, pos32[p[r].x], pos32[p[r].y], wall32[p[r].y], br.x,
-                                      pb.on ? pb.range32 : nullptr)) {
-                const uint8_t f0 = flags[k];
-                if (f0 & PF_NONZERO) {
-                    hist[k] = make_double4_32a(0.0, 0.0, 0.0, 0.0);
-                    v0[k] = 0.0;
-                }
-                if (f0 != 0) flags[k] = 0;
-            } else {
-                near = true;
+            for (int r = 0; r < PAIR_TILE; ++r) {              // (the candidates' loads overlap)
+                const uint32_t k = base + r * TPB;
+                p[r] = k < np ? sm[k] : make_uint2(0u, 0u);
+                pi[r] = k < np ? param[k] : 0u;
             }
+#pragma unroll
+            for (int r = 0; r < PAIR_TILE; ++r) {
+                const uint32_t k = base + r * TPB;
+                bool near = false;
+                if (k < np) {
+                    const float2 br = brief[pi[r]];
+                    const int cd = __float_as_int(br.y);
+                    if (cd && certainly_apart(cd, pos32[p[r].x], pos32[p[r].y], wall32[p[r].y], br.x,
+                                              pb.on ? pb.range32 : nullptr)) {
+                        const uint8_t f0 = flags[k];
+                        if (f0 & PF_NONZERO) {
+                            hist[k] = make_double4_32a(0.0, 0.0, 0.0, 0.0);
+                            v0[k] = 0.0;
+                        }
+                        if (f0 != 0) flags[k] = 0;
+                    } else {
+                        near = true;
+                    }
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, near);
+                uint32_t at = 0;
+                if (lane == 0 && m) at = atomicAdd(&count, (uint32_t)__popc(m));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (near) list[at + __popc(m & ((1u << lane) - 1u))] = k;
+            }
+            __syncthreads();
+            n = count;
+            __syncthreads();                                   // (before the next tile adds to it)
         }
-        const unsigned m = __ballot_sync(0xffffffffu, near);
-        uint32_t at = 0;
-        if (lane == 0 && m) at = atomicAdd(&count, (uint32_t)__popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (near) list[at + __popc(m & ((1u << lane) - 1u))] = k;
+        if (n == 0) return;
+        const uint32_t take = min(n, (uint32_t)TPB);
+        const bool mine = threadIdx.x < take;
+        const uint32_t k = mine ? list[n - take + threadIdx.x] : 0u;
+        n -= take;
+        __syncthreads();
+        if (threadIdx.x == 0) count = n;
+        if (mine)
+            pair_exact(k, sm, param, params, geom, hole, pos, vel, av, ox, oz, hist, v0, flags, out, dt, backup, pb,
+                       touched);
+        __syncthreads();
     }
-    __syncthreads();
-    const uint32_t nw = count;
-    for (uint32_t q = threadIdx.x; q < nw; q += TPB)
-        pair_exact(list[q], sm, param, params, geom, hole, pos, vel, av, ox, oz, hist, v0, flags, out, dt, backup, pb,
-                   touched);
 }
 
 __device__ __forceinline__ void add_entry(uint32_t ent, uint8_t f, const double* __restrict__ out, d3& J, d3& JA) {
@@ -1504,13 +1524,14 @@ int Engine::step_once(bool write_impulses) {
     // CalculateImpact
     if (prof) CK(cudaEventRecord(ev_[0], stream_));
     if (cur_.np) {
-        // Candidates per block: 2048 where that still gives a block to every SM several times over, 512
-        // for short lists.  20 steps with their rebuild, us, at 256 / 512 / 1024 / 2048 per block: the
-        // 150,000-sphere drum (about a million candidates) 9590 / 7830 / 7140 / 6900; the 8,000-sphere
-        // box (45,000) 1661 / 1522 / 1563 / 1649.
-        const uint32_t per = cur_.np >= 8u * TPB * 304u ? 8u : cur_.np >= 4u * TPB * 152u ? 4u : 2u;
-        auto k = per == 8u ? k_pair<8> : per == 4u ? k_pair<4> : k_pair<2>;
-        k<<<blocks_for(cur_.np, (int)(per * TPB)), TPB, 0, stream_>>>(
+        if (!pair_grid_) {                         // the blocks resident at once
+            int blocks = 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_pair, TPB, 0) != cudaSuccess || blocks < 1) blocks = 1;
+            int sms = 1;
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opts_.device);
+            pair_grid_ = (unsigned)(blocks * std::max(sms, 1));
+        }
+        k_pair<<<std::min(pair_grid_, blocks_for(cur_.np, PAIR_TILE * TPB)), TPB, 0, stream_>>>(
             cur_.np, cur_.sm, cur_.param, d_params_, d_geom_, d_hole_, d_brief_, d_pos_, d_vel_, d_av_, d_ox_, d_oz_,
             d_pos32_, d_wall32_, cur_.hist, cur_.v0, cur_.flags, cur_.out, dt, backup_pending_ ? 1 : 0, tab_.pbc,
             d_touched_);

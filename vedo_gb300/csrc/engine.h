@@ -138,6 +138,7 @@ private:
     float4* d_pos32_ = nullptr;
     // per object: 1 when a pair of this step applied an impulse to it (k_pair sets, k_obj clears)
     uint8_t* d_touched_ = nullptr;
+    unsigned pair_grid_ = 0;        // blocks of k_pair resident at once
     // the candidate list of LeapConsultant (else NBSConsultant), and its cell edge's largest range
     bool leap_ = false;
     double leap_rmax_ = 0.0;
