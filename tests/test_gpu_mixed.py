@@ -460,3 +460,20 @@ def test_tick_of_a_large_dense_packing(engine_lib):
             assert np.array_equal(sa[f], sb[f]), f
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("which,n,block", [("pack", 1500, 256), ("pack", 30000, 32), ("pack", 90000, 96),
+                                           ("hopper", 400, 64), ("hopper", 20000, 128), ("hopper", 60000, 192)])
+def test_deferred_spheres_spread_over_the_grid(which, n, block, engine_lib):
+    """The split tick's full half at 8 to 1 threads a deferred sphere and several rounds a block, against
+    the pair pass: identical bits."""
+    sc = scenes.dense_pack(n=n, steps=1000) if which == "pack" else scenes.hopper(n=n, seed=n, steps=1000, touching=True)
+    sc.velocity[:n] = np.random.default_rng(n).normal(0.0, 0.02, size=(n, 3))
+    a = engine_lib.GpuEngine(sc, precision=1, split_tick=True, tick_block=block)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True)
+    for k in (1, 24):
+        a.run(k)
+        b.run(k)
+        _same_run(a, b)
+    a.close()
+    b.close()

@@ -959,8 +959,8 @@ __host__ __device__ __forceinline__ uint32_t tick_slots(uint32_t spheres) {
     return spheres * SHARES_PER_SPHERE > 64u ? spheres * SHARES_PER_SPHERE : 64u;   // at least one sphere's chunk
 }
 template <int LAW, bool XS, int KIND>
-__device__ __forceinline__ void tick_item(const TickArgs& a, uint32_t base, const uint2& it, float4* share) {
-    const uint32_t e = it.x, i = base + (it.y >> 16), slot = it.y & 0xffffu;
+__device__ __forceinline__ void tick_item(const TickArgs& a, uint32_t i, const uint2& it, float4* share) {
+    const uint32_t e = it.x, slot = it.y & 0xffffu;
     const uint32_t meta = a.nmeta[e];
     const d3 Pi = XS || KIND == 2 ? mk(0.0, 0.0, 0.0) : ld(a.xA, i);
     f3 Jp, tA, tB;
@@ -970,18 +970,17 @@ __device__ __forceinline__ void tick_item(const TickArgs& a, uint32_t base, cons
     share[2 * slot] = make_float4(Ji.x, Ji.y, Ji.z, __int_as_float(app));
     share[2 * slot + 1] = make_float4(ti.x, ti.y, ti.z, 0.0f);
 }
+// One block's spheres: count of them from `base` on (list == nullptr), or those the list names.  Returns
+// the thread's squared speed bounds.
 template <int LAW, bool XS>
-__global__ void __launch_bounds__(TPB, 2) k_tick(TickArgs a, int lanes) {
+__device__ __forceinline__ float2 tick_block(const TickArgs& a, int lanes, uint32_t base, uint32_t count,
+                                             const uint32_t* __restrict__ list) {
     extern __shared__ float4 share[];              // [2 * slots], then the slots' items
     __shared__ uint32_t pk[TPB + 1], warp_tot[TPB / 32];
     __shared__ uint8_t note[TPB];                  // per sphere: 1 stepped, 2 quiet, 4 frozen, 8 no clean walk, count << 4
-    step_order();
     const uint32_t t = threadIdx.x, B = blockDim.x >> lanes, G = 1u << lanes;
-    const uint32_t s = t >> lanes, g = t & (G - 1u), base = blockIdx.x * B;
-    if (held_step(a)) {                            // the same value for every thread of the launch
-        if (t < B) hold_state(a, base + t);
-        return;
-    }
+    const uint32_t s = t >> lanes, g = t & (G - 1u);
+    auto sphere = [&](uint32_t q) { return q >= count ? a.n : list ? list[base + q] : base + q; };
     const uint32_t slots = tick_slots(B);
     uint2* items = reinterpret_cast<uint2*>(share + 2 * slots);
     const int lane = (int)(t & 31u);
@@ -991,13 +990,13 @@ __global__ void __launch_bounds__(TPB, 2) k_tick(TickArgs a, int lanes) {
     const float* L = nullptr;
     bool walk = false, reset = false;
     {
-        const uint32_t i = base + s;
+        const uint32_t i = sphere(s);
         uint8_t nt = 0;
         if (i < a.n) {
             const ModelDev& M = a.models[a.model_of[i]];
             const SceneDev& S = a.scenes[a.scene_of[i]];
             if (M.scope == SCOPE_LOCAL && S.active) {
-                const uint32_t qc = a.qcnt[i];
+                const uint32_t qc = a.work ? 0u : a.qcnt[i];   // (kept by the light tick when there is one)
                 const float2 cl = a.clear[i];
                 pad = 2.0f * a.disp[0];
                 const bool quiet = qc >= 2u && !a.write_imp && pad <= cl.x && a.disp[1] <= cl.y;
@@ -1079,9 +1078,9 @@ __global__ void __launch_bounds__(TPB, 2) k_tick(TickArgs a, int lanes) {
                                            s << 16 | (slot_of(s) - first + (uint32_t)__popcll(full & below)));
                 }
             __syncthreads();
-            for (uint32_t q = t; q < nP; q += blockDim.x) tick_item<LAW, XS, 1>(a, base, items[q], share);
+            for (uint32_t q = t; q < nP; q += blockDim.x) tick_item<LAW, XS, 1>(a, sphere(items[q].y >> 16), items[q], share);
             for (uint32_t q = blockDim.x - 1u - t; q < nW; q += blockDim.x)
-                tick_item<LAW, XS, 2>(a, base, items[nP + q], share);
+                tick_item<LAW, XS, 2>(a, sphere(items[nP + q].y >> 16), items[nP + q], share);
             __syncthreads();
             if (t >= s0 && t < s1)
                 for (uint32_t q = slot_of(t) - first; q < slot_of(t + 1u) - first; ++q) {
@@ -1102,19 +1101,30 @@ __global__ void __launch_bounds__(TPB, 2) k_tick(TickArgs a, int lanes) {
     __syncthreads();
     float2 vmax_local = make_float2(0.0f, 0.0f);
     if (t < B) {
-        const uint32_t i = base + t, nt = note[t];
+        const uint32_t i = sphere(t), nt = note[t];
         if (nt & 1u) {
             const bool quiet = nt & 2u;
             const uint32_t mi = a.model_of[i];
-            if (!quiet) note_walk(a, i, nt >> 4, nt & 8u);
+            if (!quiet && !a.work) note_walk(a, i, nt >> 4, nt & 8u);
             vmax_local = finish_sphere<XS>(a, i, a.models[mi].behavior == BEH_MOBILE, quiet, a.scenes[a.scene_of[i]],
                                            ld(a.xA, i), ld(a.v64, i), a.mf[2 * mi], a.mf[2 * mi + 1], J, JA);
         } else if (nt & 4u) {
             hold_state(a, i);
         }
     }
-    reduce_vmax(a, vmax_local);
+    return vmax_local;
 }
+template <int LAW, bool XS>
+__global__ void __launch_bounds__(TPB, 2) k_tick(TickArgs a, int lanes) {
+    step_order();
+    const uint32_t B = blockDim.x >> lanes, base = blockIdx.x * B;
+    if (held_step(a)) {                            // the same value for every thread of the launch
+        if (threadIdx.x < B) hold_state(a, base + threadIdx.x);
+        return;
+    }
+    reduce_vmax(a, tick_block<LAW, XS>(a, lanes, base, min(B, a.n - base), nullptr));
+}
+
 
 // The full tick with one thread per sphere, for large dense packings (launch_tick's rule): there the
 // shared slots above overflow and cost the gathers their cache, and every lane has pairs anyway.
@@ -1131,10 +1141,37 @@ __global__ void __launch_bounds__(TPB) k_tick_each(TickArgs a) {
     reduce_vmax(a, vmax_local);
 }
 
-// The full tick of the split tick: a grid sized to the resident threads strides over the
-// spheres the light kernel deferred (none in a held step).
+// Threads per sphere of the full tick, as a power of two: 8 or 4 while that keeps every sphere resident
+// at once (`room` threads), 2 to five eighths of that many spheres, then 1 (launch_tick has the times).
+__host__ __device__ __forceinline__ int tick_lanes(uint64_t spheres, uint64_t room) {
+    int lanes = 8u * spheres <= 5u * room ? 1 : 0;
+    while (lanes >= 1 && lanes < 3 && (spheres << (lanes + 1)) <= room) ++lanes;
+    return lanes;
+}
+
+// The full tick of the split tick: a grid of the resident size takes the spheres the light kernel
+// deferred (none in a held step), spread over its threads as the full tick spreads a scene of that many.
+// (With one thread to a deferred sphere a 30,000-sphere hopper's step was 88 us, 2,000 packed spheres'
+// 95; 55 and 40 like this.)
 template <int LAW, bool XS>
-__global__ void __launch_bounds__(TPB) k_tick_work(TickArgs a) {
+__global__ void __launch_bounds__(TPB, 2) k_tick_work(TickArgs a) {
+    step_order();
+    float2 vmax_local = make_float2(0.0f, 0.0f);
+    if (!held_step(a)) {
+        const uint32_t nw = *a.nwork;
+        const int lanes = tick_lanes(nw, (uint64_t)gridDim.x * blockDim.x);
+        const uint32_t B = blockDim.x >> lanes;
+        for (uint32_t base = blockIdx.x * B; base < nw; base += gridDim.x * B) {
+            vmax_local = fmax2(vmax_local, tick_block<LAW, XS>(a, lanes, base, min(B, nw - base), a.work));
+            __syncthreads();                       // (the shared arrays, for the next spheres)
+        }
+    }
+    reduce_vmax(a, vmax_local);
+}
+
+// ... and with a thread per deferred sphere, for large dense packings (launch_work's rule).
+template <int LAW, bool XS>
+__global__ void __launch_bounds__(TPB) k_tick_work_each(TickArgs a) {
     step_order();
     float2 vmax_local = make_float2(0.0f, 0.0f);
     if (!held_step(a)) {
@@ -2924,6 +2961,7 @@ private:
     }
     int rebuild();
     void launch_step(bool write_imp);
+    cudaError_t launch_work(bool dep, void (*k)(TickArgs), void (*each)(TickArgs), const TickArgs& a);
     cudaError_t launch_tick(bool dep, void (*k)(TickArgs, int), void (*each)(TickArgs), const TickArgs& a);
     cudaError_t launch_err_ = cudaSuccess;   // the first failed launch of the step kernels
     int step_chunk(uint32_t chunk, bool imp_last, float* use_after);
@@ -3900,6 +3938,28 @@ static cudaError_t step_launch(bool dep, void (*k)(P...), unsigned grid, unsigne
     return step_launch_smem(dep, k, grid, block, 0, s, args...);
 }
 
+// The dynamic shared memory of a tick block of `spheres`, granted to kernel k.
+static cudaError_t tick_smem(const void* k, unsigned spheres, size_t* bytes) {
+    *bytes = (size_t)tick_slots(spheres) * (2 * sizeof(float4) + sizeof(uint2));
+    return *bytes > 48 * 1024 ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*bytes)
+                              : cudaSuccess;
+}
+// The split tick's full half over the deferred spheres: blocks of at most 128 threads, resident at once.
+// More spheres than resident threads with lists of ten entries and more: a thread per sphere (100,000 and
+// 300,000 packed spheres 145 and 285 us a step, 153 and 314 spread out; a hopper of 100,000 spread out 106
+// against 130).
+cudaError_t MixedEngine::launch_work(bool dep, void (*k)(TickArgs), void (*each)(TickArgs), const TickArgs& a) {
+    if (n_ > (uint32_t)sms_ * 512u && nl_[nlc_].ne >= 10ull * n_)
+        return step_launch(dep, each, std::min<unsigned>((unsigned)((n_ + tpb_ - 1) / tpb_), (unsigned)sms_ * 512u / (unsigned)tpb_),
+                           (unsigned)tpb_, stream_, a);
+    const unsigned block = tpb_ > 128 && tpb_ % 64 == 0 ? 128u : (unsigned)tpb_;
+    size_t bytes = 0;
+    const cudaError_t e = tick_smem((const void*)k, block, &bytes);
+    if (e != cudaSuccess) return e;
+    const unsigned grid = std::min<unsigned>((n_ + block - 1u) / block * 8u, (unsigned)sms_ * 512u / block);
+    return step_launch_smem(dep, k, std::max(grid, 1u), block, bytes, stream_, a);
+}
+
 // The full tick's launch.  Threads per sphere: 8 or 4 while that keeps every sphere of the scene resident
 // at once (512 threads an SM at the tick's registers), 2 to five eighths of that many spheres, then 1, in
 // blocks of at most 128.  us per step at 1 / 2 / 4 / 8 (GB300): 8,000-sphere box 37 / 29 / 26 / 24; 10,000
@@ -3913,24 +3973,20 @@ cudaError_t MixedEngine::launch_tick(bool dep, void (*k)(TickArgs, int), void (*
     const uint64_t room = (uint64_t)sms_ * 512u;
     if (2ull * n_ > 5u * room && nl_[nlc_].ne >= 10ull * n_)
         return step_launch(dep, each, (unsigned)((n_ + tpb_ - 1) / tpb_), (unsigned)tpb_, stream_, a);
-    int lanes = 8ull * n_ <= 5u * room ? 1 : 0;
-    while (lanes >= 1 && lanes < 3 && ((uint64_t)n_ << (lanes + 1)) <= room) ++lanes;
+    const int lanes = tick_lanes(n_, room);
     unsigned block = (unsigned)tpb_;
     while (block >= 128u && block % 64u == 0u &&
            (((uint64_t)n_ << lanes) < (uint64_t)sms_ * block || (lanes == 0 && block > 128u)))
         block /= 2u;
     const unsigned spheres = block >> lanes;
-    const size_t bytes = (size_t)tick_slots(spheres) * (2 * sizeof(float4) + sizeof(uint2));
-    if (bytes > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return e;
-    }
+    size_t bytes = 0;
+    const cudaError_t e = tick_smem((const void*)k, spheres, &bytes);
+    if (e != cudaSuccess) return e;
     return step_launch_smem(dep, k, (n_ + spheres - 1u) / spheres, block, bytes, stream_, a, lanes);
 }
 
 void MixedEngine::launch_step(bool write_imp) {
     TickArgs a = args(write_imp);
-    const unsigned nb = (unsigned)((n_ + tpb_ - 1) / tpb_);
     cudaEvent_t* pe = nullptr;
     if (profiling_ && pev_used_ + 3 <= pev_.size()) {
         pe = &pev_[pev_used_];
@@ -3944,7 +4000,6 @@ void MixedEngine::launch_step(bool write_imp) {
     auto note = [&](cudaError_t e) {
         if (e != cudaSuccess && launch_err_ == cudaSuccess) launch_err_ = e;
     };
-    unsigned nb_full = nb;
     if (pair_pass_) {               // prefilter pass, pair pass over its worklist, per-sphere sums
         // (the worklist count is zeroed by k_walls at the end of every step)
         note(step_launch(dep, k_tick_pf, nblk(n_), TPB, stream_, a));
@@ -3982,13 +4037,11 @@ void MixedEngine::launch_step(bool write_imp) {
         // (the worklist count is zeroed by k_walls at the end of every step)
         note(step_launch(dep, xs_stored_ ? k_tick_light<true> : k_tick_light<false>, nblk(n_), TPB, stream_, a));
         ++launches_;
-        // the full tick at its residency (128 registers: 16 warps per SM) strides over the worklist
-        nb_full = std::min<unsigned>(nb, (unsigned)sms_ * 512u / (unsigned)tpb_);
     }
 #define VEDO_TICK(L)                                                                                        \
     if (split_tick_)                                                                                        \
-        note(step_launch(dep, xs_stored_ ? k_tick_work<L, true> : k_tick_work<L, false>, nb_full,            \
-                         (unsigned)tpb_, stream_, a));                                                       \
+        note(launch_work(dep, xs_stored_ ? k_tick_work<L, true> : k_tick_work<L, false>,                      \
+                         xs_stored_ ? k_tick_work_each<L, true> : k_tick_work_each<L, false>, a));            \
     else                                                                                                    \
         note(launch_tick(dep, xs_stored_ ? k_tick<L, true> : k_tick<L, false>,                              \
                          xs_stored_ ? k_tick_each<L, true> : k_tick_each<L, false>, a))
