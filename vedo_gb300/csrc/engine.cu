@@ -257,17 +257,25 @@ __global__ void __launch_bounds__(TPB, 3) k_pair(uint32_t np, const uint2* __res
     }
 }
 
-__device__ __forceinline__ void add_entry(uint32_t ent, uint8_t f, const double* __restrict__ out, d3& J, d3& JA) {
-    if (!(f & PF_APPLIED)) return;
+// An entry's share of its object: the slave's A->AddImpact(ImpactA, tA), the master's
+// B->AddImpact(-1.0 * ImpactA, tB); a law without torques adds none.
+struct Share {
+    d3 J, T;
+    bool angular;
+};
+__device__ __forceinline__ Share load_share(uint32_t ent, uint8_t f, const double* __restrict__ out) {
     const double* o = out + 9 * (size_t)(ent >> 1);
-    const d3 Jk = mk(o[0], o[1], o[2]);
-    if (ent & 1) {                                            // master: B->AddImpact(-1.0 * ImpactA, tB)
-        J = add(J, neg(Jk));
-        if (f & PF_ANGULAR) JA = add(JA, mk(o[6], o[7], o[8]));
-    } else {                                                  // slave: A->AddImpact(ImpactA, tA)
-        J = add(J, Jk);
-        if (f & PF_ANGULAR) JA = add(JA, mk(o[3], o[4], o[5]));
-    }
+    Share s;
+    s.J = mk(o[0], o[1], o[2]);
+    if (ent & 1) s.J = neg(s.J);
+    s.angular = f & PF_ANGULAR;
+    const double* t = o + (ent & 1 ? 6 : 3);
+    s.T = s.angular ? mk(t[0], t[1], t[2]) : mk(0.0, 0.0, 0.0);
+    return s;
+}
+__device__ __forceinline__ void add_share(const Share& s, d3& J, d3& JA) {
+    J = add(J, s.J);
+    if (s.angular) JA = add(JA, s.T);
 }
 
 // FP32 copies used by the prefilters: position relative to `origin`, and for plates and
@@ -342,6 +350,7 @@ struct ObjArgs {
     uint8_t* touched;
     uint32_t nglob;
     const uint32_t* glob;
+    uint32_t per;                      // local objects a block takes, a multiple of 32
 };
 
 // One block per scope-global object, when its sum is wanted (its impulse is written, or it responds):
@@ -411,14 +420,16 @@ __device__ __forceinline__ void global_object(const ObjArgs& a, uint32_t i) {
 }
 
 // The first nglob blocks take the scope-global objects (no object reads another's state here, so the
-// two run side by side in one launch), the others the local objects, one per thread.
+// two run side by side in one launch), the others `per` local objects each, one per thread: FP64 work,
+// which a short array spreads over as many SMs as it can (20 steps with their rebuild of 8,000 spheres:
+// 1260 us in 32 full blocks, the FP64 pipes of 32 SMs, 1182 in 250 blocks of 32 objects).
 __global__ void __launch_bounds__(TPB) k_obj(ObjArgs a) {
     if (blockIdx.x < a.nglob) {
         global_object(a, a.glob[blockIdx.x]);
         return;
     }
-    const uint32_t i = (blockIdx.x - a.nglob) * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
+    const uint32_t i = (blockIdx.x - a.nglob) * a.per + threadIdx.x;
+    if (threadIdx.x >= a.per || i >= a.n) return;
     const ModelDev& m = a.models[a.model_of[i]];
     if (m.scope == SCOPE_GLOBAL) return;
     d3 J = mk(0.0, 0.0, 0.0), JA = mk(0.0, 0.0, 0.0);
@@ -428,18 +439,32 @@ __global__ void __launch_bounds__(TPB) k_obj(ObjArgs a) {
         const uint32_t e0 = a.csr_ptr[i], e1 = a.csr_ptr[i + 1];
         // the entries that applied an impulse are marked first (integer work), then summed in entry
         // order: a warp issues each FP64 add once per marked entry of its busiest object, not once
-        // per candidate entry (most candidates of an object apply nothing)
-        const uint32_t c1 = min(e1, e0 + 64u);
-        unsigned long long mark = 0ull;
-        for (uint32_t e = e0; e < c1; ++e)
-            if (a.flags[a.csr_ent[e] >> 1] & PF_APPLIED) mark |= 1ull << (e - e0);
-        for (; mark; mark &= mark - 1) {
-            const uint32_t ent = a.csr_ent[e0 + (uint32_t)(__ffsll(mark) - 1)];
-            add_entry(ent, a.flags[ent >> 1], a.out, J, JA);
-        }
-        for (uint32_t e = c1; e < e1; ++e) {                   // long lists: the entries after 64
-            const uint32_t ent = a.csr_ent[e];
-            add_entry(ent, a.flags[ent >> 1], a.out, J, JA);
+        // per candidate entry.  Flags are loaded eight entries at a time and shares two, or each use waits
+        // for its own load
+        for (uint32_t c0 = e0; c0 < e1; c0 += 64u) {
+            const uint32_t c1 = min(e1, c0 + 64u);
+            unsigned long long mark = 0ull;
+            for (uint32_t e = c0; e < c1; e += 8u) {
+                uint32_t ent[8];
+                uint8_t f[8];
+#pragma unroll
+                for (uint32_t u = 0; u < 8u; ++u) ent[u] = e + u < c1 ? a.csr_ent[e + u] : 0u;
+#pragma unroll
+                for (uint32_t u = 0; u < 8u; ++u) f[u] = e + u < c1 ? a.flags[ent[u] >> 1] : (uint8_t)0;
+#pragma unroll
+                for (uint32_t u = 0; u < 8u; ++u)
+                    mark |= (unsigned long long)(f[u] & PF_APPLIED ? 1u : 0u) << ((e - c0 + u) & 63u);
+            }
+            while (mark) {
+                const uint32_t ea = a.csr_ent[c0 + (uint32_t)(__ffsll((long long)mark) - 1)];
+                mark &= mark - 1;
+                const bool two = mark != 0ull;
+                const uint32_t eb = two ? a.csr_ent[c0 + (uint32_t)(__ffsll((long long)mark) - 1)] : ea;
+                mark &= mark - 1;
+                const Share sa = load_share(ea, a.flags[ea >> 1], a.out), sb = load_share(eb, a.flags[eb >> 1], a.out);
+                add_share(sa, J, JA);
+                if (two) add_share(sb, J, JA);
+            }
         }
     }
     finish_object(i, m, J, JA, a.dt, a.fimp, a.pos, a.vel, a.av, a.ox, a.oz, a.imp, a.aimp, a.write_imp, a.origin,
@@ -953,9 +978,30 @@ __global__ void __launch_bounds__(TPB) k_setup(uint32_t np, uint32_t per, const 
     }
 }
 
+// Where each object's entries begin in the sorted keys.  BY_KEY: a thread per entry marks the objects
+// between its key and the one before it (with fewer entries than objects, or above a million, a thread
+// per object searches; 8,000 objects of 34 entries: 9.6 us searched, 3.2 marked; 150,000 of 44: 13, 18).
+template <bool BY_KEY>
 __global__ void __launch_bounds__(TPB) k_csr_ptr(uint32_t n, const uint32_t* __restrict__ key, uint32_t m,
                                                  uint32_t* __restrict__ ptr) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (BY_KEY) {
+        uint32_t q0 = 1u, q1 = 0u;                             // objects [q0, q1] begin at entry i
+        if (i <= m) {
+            q0 = i ? key[i - 1] + 1u : 0u;
+            q1 = i < m ? key[i] : n;
+        }
+        const bool wide = q0 + 32u < q1;                        // a long gap: the warp fills it
+        if (!wide)
+            for (uint32_t q = q0; q <= q1; ++q) ptr[q] = i;
+        for (unsigned w = __ballot_sync(0xffffffffu, wide); w; w &= w - 1u) {
+            const int l = __ffs((int)w) - 1;
+            const uint32_t a = __shfl_sync(0xffffffffu, q0, l), b = __shfl_sync(0xffffffffu, q1, l),
+                           at = __shfl_sync(0xffffffffu, i, l);
+            for (uint32_t q = a + (threadIdx.x & 31u); q <= b; q += 32u) ptr[q] = at;
+        }
+        return;
+    }
     if (i > n) return;
     uint32_t lo = 0, hi = m;
     while (lo < hi) {
@@ -1504,7 +1550,8 @@ int Engine::rebuild(bool from_records) {
         ++own;
         CK(radix_sort_u32(d_ck_, cur_.csr_ent, d_ck_alt_, d_cv_alt_, m, 0, obits, scratch_, stream_, calt));
     }
-    k_csr_ptr<<<blocks_for((uint64_t)n_ + 1), TPB, 0, stream_>>>(n_, d_ck_, m, cur_.csr_ptr);
+    if (m >= n_ && m <= (1u << 20)) k_csr_ptr<true><<<blocks_for((uint64_t)m + 1), TPB, 0, stream_>>>(n_, d_ck_, m, cur_.csr_ptr);
+    else k_csr_ptr<false><<<blocks_for((uint64_t)n_ + 1), TPB, 0, stream_>>>(n_, d_ck_, m, cur_.csr_ptr);
     ++own;
     CK(cudaGetLastError());
     launches_ += own + (g_sort_scan_launches - l0);
@@ -1562,7 +1609,8 @@ int Engine::step_once(bool write_impulses) {
     oa.touched = d_touched_;
     oa.nglob = (uint32_t)global_ids_.size();
     oa.glob = d_global_;
-    k_obj<<<oa.nglob + blocks_for(n_), TPB, 0, stream_>>>(oa);
+    oa.per = std::min<uint32_t>(TPB, std::max(32u, (n_ / 608u + 31u) / 32u * 32u));   // four blocks an SM
+    k_obj<<<oa.nglob + blocks_for(n_, (int)oa.per), TPB, 0, stream_>>>(oa);
     ++launches_;
     if (prof) CK(cudaEventRecord(ev_[2], stream_));
     backup_pending_ = true;
