@@ -2991,6 +2991,8 @@ private:
     // profiling (+2), with the impulse output of a call's last step (+4)
     cudaGraphExec_t graph_[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     uint64_t graph_launches_[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint32_t graph_chunks_[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // intervals of the kind launched plainly on this list
+    bool capture_now_ = false;      // capture at once (the autotuner times replayed graphs)
     unsigned ev_flags_ = cudaEventRecordDefault;      // cudaEventRecordExternal while capturing
     std::vector<cudaEvent_t> pev_;  // profiling: per step, events before the tick, after it, after the walls
     uint32_t pev_used_ = 0;
@@ -3199,6 +3201,7 @@ void MixedEngine::drop_graphs() {
         if (g) cudaGraphExecDestroy(g);
         g = nullptr;
     }
+    for (auto& c : graph_chunks_) c = 0;
 }
 
 void MixedEngine::set_skin(float frac) {
@@ -4145,9 +4148,12 @@ int MixedEngine::launch_persistent(uint32_t chunk) {
     return 0;
 }
 
-// `chunk` steps, then one read of the displacement bound and of the held-step count.  A full
-// check interval without impulse output replays a CUDA graph captured once per list, or runs as
-// one persistent launch.
+// `chunk` steps, then one read of the displacement bound and of the held-step count.  A full check
+// interval runs as one persistent launch, or replays a CUDA graph captured once per list when the list
+// has served GRAPH_AFTER intervals of its kind: capturing and instantiating the graph of ten steps costs
+// about 200 us, and replaying it saves about 10 us an interval over plain launches, so a list that is
+// rebuilt after a few intervals (spheres at speed, a call of a few steps at a time) would only pay for it.
+constexpr uint32_t GRAPH_AFTER = 12;
 int MixedEngine::step_chunk(uint32_t chunk, bool imp_last, float* use_after) {
     const uint32_t ci = opts_.check_interval;
     if (profiling_ && pev_.size() < 3 * (size_t)ci) {
@@ -4165,9 +4171,9 @@ int MixedEngine::step_chunk(uint32_t chunk, bool imp_last, float* use_after) {
     }
     if (persisted == 0) {
         // (launched)
-    } else if (opts_.graphs && chunk == ci) {
-        const int c0 = cur_;
-        const int gi = c0 + (profiling_ ? 2 : 0) + (imp_last ? 4 : 0);
+    } else if (const int gk = cur_ + (profiling_ ? 2 : 0) + (imp_last ? 4 : 0);
+               opts_.graphs && chunk == ci && (graph_[gk] || capture_now_ || ++graph_chunks_[gk] > GRAPH_AFTER)) {
+        const int c0 = cur_, gi = gk;
         if (!graph_[gi]) {
             cudaGraph_t g = nullptr;
             const uint64_t l0 = launches_;
@@ -4250,6 +4256,11 @@ int MixedEngine::step_chunk(uint32_t chunk, bool imp_last, float* use_after) {
 // expected to last at the displacement growth just measured.
 int MixedEngine::autotune(uint32_t max_steps, uint32_t* taken) {
     *taken = 0;
+    struct Eager {                                   // the trials time replayed graphs from their first interval on
+        bool& on;
+        explicit Eager(bool& f) : on(f) { on = true; }
+        ~Eager() { on = false; }
+    } eager(capture_now_);
     const uint32_t ci = opts_.check_interval;
     const int blocks[] = {64, 128, 256};
     const float skins[] = {0.05f, 0.1f, 0.15f, 0.25f, 0.4f};
