@@ -1710,10 +1710,17 @@ __global__ void k_pack3(uint32_t n, const double* __restrict__ src, double4_32a*
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = make_double4_32a(src[3 * (size_t)i], src[3 * (size_t)i + 1], src[3 * (size_t)i + 2], 0.0);
 }
-__global__ void k_unpack3(uint32_t n, const double4_32a* __restrict__ src, double* __restrict__ dst) {
+// Every array asked for in one launch (blockIdx.y), as a call of a few dozen objects is made of its
+// launches.
+struct Fields {
+    const double4_32a* src[7];
+    double* dst[7];
+};
+__global__ void k_unpack3(uint32_t n, Fields f) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        const double4_32a v = src[i];
+        const double4_32a v = f.src[blockIdx.y][i];
+        double* dst = f.dst[blockIdx.y];
         dst[3 * (size_t)i] = v.x;
         dst[3 * (size_t)i + 1] = v.y;
         dst[3 * (size_t)i + 2] = v.z;
@@ -1733,12 +1740,17 @@ int Engine::get_state(const vedo_state_view& v) {
     double* dst[] = {v.position, v.velocity, v.angular_velocity, v.orientation_x, v.orientation_z, v.impact,
                      v.angular_impact};
     const double4_32a* src[] = {d_pos_, d_vel_, d_av_, d_ox_, d_oz_, d_imp_, d_aimp_};
+    Fields f{};
+    int nf = 0;
     for (int k = 0; k < 7; ++k) {
         if (!dst[k]) continue;
-        double* st = d_stage_ + (size_t)k * 3 * n_;
-        k_unpack3<<<blocks_for(n_), TPB, 0, stream_>>>(n_, src[k], st);
-        CK(cudaMemcpyAsync(dst[k], st, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
+        f.src[nf] = src[k];
+        f.dst[nf++] = d_stage_ + (size_t)k * 3 * n_;
     }
+    if (nf) k_unpack3<<<dim3(blocks_for(n_), (unsigned)nf), TPB, 0, stream_>>>(n_, f);
+    for (int k = 0; k < 7; ++k)
+        if (dst[k])
+            CK(cudaMemcpyAsync(dst[k], d_stage_ + (size_t)k * 3 * n_, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
     CK(cudaGetLastError());
     return VEDO_OK;

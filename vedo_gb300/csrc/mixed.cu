@@ -2585,11 +2585,17 @@ __global__ void __launch_bounds__(TPB) k_place(uint32_t n, const double* __restr
 }
 // n objects of the caller's order starting at `off` into [n][3] doubles: object off + i is
 // stored at int_of[off + i]
+// (every array asked for in one launch, blockIdx.y)
+struct Fields {
+    const double4_32a* src[7];
+    double* dst[7];
+};
 __global__ void __launch_bounds__(TPB) k_unpack3m(uint32_t n, uint32_t off, const uint32_t* __restrict__ int_of,
-                                                  const double4_32a* __restrict__ src, double* __restrict__ dst) {
+                                                  Fields f) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        const double4_32a v = src[int_of[off + i]];
+        const double4_32a v = f.src[blockIdx.y][int_of[off + i]];
+        double* dst = f.dst[blockIdx.y];
         dst[3 * (size_t)i] = v.x;
         dst[3 * (size_t)i + 1] = v.y;
         dst[3 * (size_t)i + 2] = v.z;
@@ -3561,12 +3567,17 @@ int MixedEngine::get_state_slice(uint32_t off, uint32_t cnt, const vedo_state_vi
     double* dst[] = {v.position, v.velocity, v.angular_velocity, v.orientation_x, v.orientation_z, v.impact,
                      v.angular_impact};
     const double4_32a* src[] = {d_x_[cur_], d_v64_, d_w64_, d_ox_, d_oz_, d_imp_, d_aimp_};
+    Fields f{};
+    int nf = 0;
     for (int k = 0; k < 7; ++k) {
-        if (!dst[k] || !cnt) continue;
-        double* stg = d_stage_ + (size_t)k * 3 * n_;
-        k_unpack3m<<<nblk(cnt), TPB, 0, stream_>>>(cnt, off, d_int_of_, src[k], stg);
-        MCK(cudaMemcpyAsync(dst[k], stg, 24 * (size_t)cnt, cudaMemcpyDeviceToHost, stream_));
+        if (!dst[k]) continue;
+        f.src[nf] = src[k];
+        f.dst[nf++] = d_stage_ + (size_t)k * 3 * n_;
     }
+    if (nf && cnt) k_unpack3m<<<dim3(nblk(cnt), (unsigned)nf), TPB, 0, stream_>>>(cnt, off, d_int_of_, f);
+    for (int k = 0; k < 7; ++k)
+        if (dst[k] && cnt)
+            MCK(cudaMemcpyAsync(dst[k], d_stage_ + (size_t)k * 3 * n_, 24 * (size_t)cnt, cudaMemcpyDeviceToHost, stream_));
     MCK(cudaStreamSynchronize(stream_));
     MCK(cudaGetLastError());
     return VEDO_OK;
@@ -4489,12 +4500,17 @@ int MixedEngine::get_state(const vedo_state_view& v) {
     double* dst[] = {v.position, v.velocity, v.angular_velocity, v.orientation_x, v.orientation_z, v.impact,
                      v.angular_impact};
     const double4_32a* src[] = {d_x_[cur_], d_v64_, d_w64_, d_ox_, d_oz_, d_imp_, d_aimp_};
+    Fields f{};
+    int nf = 0;
     for (int k = 0; k < 7; ++k) {
         if (!dst[k]) continue;
-        double* st = d_stage_ + (size_t)k * 3 * n_;
-        k_unpack3m<<<nblk(n_), TPB, 0, stream_>>>(n_, 0u, d_int_of_, src[k], st);
-        MCK(cudaMemcpyAsync(dst[k], st, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
+        f.src[nf] = src[k];
+        f.dst[nf++] = d_stage_ + (size_t)k * 3 * n_;
     }
+    if (nf && n_) k_unpack3m<<<dim3(nblk(n_), (unsigned)nf), TPB, 0, stream_>>>(n_, 0u, d_int_of_, f);
+    for (int k = 0; k < 7; ++k)
+        if (dst[k] && n_)
+            MCK(cudaMemcpyAsync(dst[k], d_stage_ + (size_t)k * 3 * n_, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
     MCK(cudaStreamSynchronize(stream_));
     MCK(cudaGetLastError());
     return VEDO_OK;
