@@ -166,7 +166,8 @@ typedef struct vedo_engine_opts {
                                  not depend on them); read the choice with
                                  vedo_gpu_get_tuning                                    */
     uint32_t graphs;          /* MIXED only: 1 = each check interval of steps is replayed
-                                 as one CUDA graph, captured once per neighbour list (default) */
+                                 as one CUDA graph, captured once per neighbour list that has
+                                 served a dozen intervals (default)                      */
     uint32_t stored_splits;   /* MIXED only: 1 = the hi/lo FP32 splits of the positions used by
                                  the sphere-pair overlap test are stored once per step; 0 = formed
                                  per pair (identical results; the autotuner chooses)       */
