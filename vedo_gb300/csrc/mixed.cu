@@ -2487,9 +2487,13 @@ __global__ void k_wall_fin(uint32_t nglob, const uint32_t* __restrict__ glob, co
 
 // Contact activity of every owner entry at the current positions (for queries): the FP64 detectors'
 // decision.  FP64 arithmetic is what bounded this pass (290 us for 500,000 packed spheres), so it is
-// kept to the pairs that need it: a sphere pair's overlap is tested in double-float with the tick's
-// tie band, and a wall's detector runs only within reach (the prefilter's test at the current
-// positions).
+// kept to the pairs that need it: a sphere pair's overlap is tested in double-float, and within the band
+// around a tie that the double-float error cannot leave the reference's formula decides; a wall's
+// detector runs only within reach (the prefilter's test at the current positions).  The band: the tick's
+// 1e-9 R^2, and 1e-13 R of the two positions' magnitudes M.  A split rounds each coordinate by 2^-48 of
+// it and their difference twice more, so |d|^2 is off by up to 2 |d| 3 2^-48 M, which is 4.3e-14 R M to
+// |d| = 2 R; beyond, R^2 - |d|^2 is clear of that error while M stays below 1e12 R.  Scenes farther out,
+// and radius sums whose squares FP32 cannot hold, take the formula.
 __global__ void __launch_bounds__(TPB) k_active(uint32_t n, TickArgs a, uint8_t* __restrict__ act) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -2501,6 +2505,7 @@ __global__ void __launch_bounds__(TPB) k_active(uint32_t n, TickArgs a, uint8_t*
     split32(Pi.x, hi_i.x, lo_i.x);
     split32(Pi.y, hi_i.y, lo_i.y);
     split32(Pi.z, hi_i.z, lo_i.z);
+    const float mag_i = l1(hi_i) + (S.pb.on ? S.pb.range32[0] + S.pb.range32[1] + S.pb.range32[2] : 0.0f);
     for (uint32_t e = e0; e < e1; ++e) {
         const uint32_t meta = a.nmeta[e];
         bool active = false;
@@ -2524,9 +2529,10 @@ __global__ void __launch_bounds__(TPB) k_active(uint32_t n, TickArgs a, uint8_t*
                 const dfl s2 = df_add(df_add(df_sq(dx), df_sq(dy)), df_sq(dz));
                 const float4 rq = a.rr32[pi];            // R^2 hi, R^2 lo, band, R
                 const dfl num = df_add(dfl{rq.x, rq.y}, dfl{-s2.hi, -s2.lo});
-                if (num.hi < -rq.z || num.hi > rq.z) {
+                const float band = rq.z + 1e-13f * rq.w * (mag_i + l1(hj));
+                if (rq.w > 1e-15f && band < 0.1f * rq.x && (num.hi < -band || num.hi > band)) {
                     active = num.hi > 0.0f;
-                } else {                                 // tie band: the reference's formula decides
+                } else {
                     const bool i_slave = meta & META_SLAVE;
                     active = tie_depth(a, pi, i_slave ? i : j, i_slave ? j : i, S.pb) > 0.0;
                 }
