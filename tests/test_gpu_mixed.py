@@ -477,3 +477,30 @@ def test_deferred_spheres_spread_over_the_grid(which, n, block, engine_lib):
         _same_run(a, b)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,block", [(31, 256), (700, 64), (20000, 32), (38912, 64), (38913, 64), (60000, 256),
+                                     (330000, 32)])
+def test_wall_pairs_spread_over_the_blocks_and_in_chunks(n, block, engine_lib):
+    """A flat layer of n spheres pressed into the floor, clear of each other: n wall pairs, fewer than the
+    wall-pair kernel has threads (a warp to each block in turn), as many, and more (taken chunk by
+    chunk, of one round of pairs and of several): the pair pass against the full tick, identical bits."""
+    r, side = 1e-3, int(np.ceil(np.sqrt(n)))
+    sc = scenes.dense_pack(n=n, radius=r, steps=1000)
+    wm, widx, wp, wox, woz = scenes.box_walls(2.2 * r * side + 8 * r, 8 * r, 1e-3)
+    k = np.arange(n)
+    sc.models[1:] = wm
+    sc.position[:n] = np.stack([2.2 * r * (k % side - 0.5 * (side - 1)), 2.2 * r * (k // side - 0.5 * (side - 1)),
+                                np.full(n, r * (1.0 - 1e-6))], 1)
+    sc.position[n:] = wp
+    sc.velocity[:n] = np.random.default_rng(n).normal(0.0, 1e-3, size=(n, 3))
+    a = engine_lib.GpuEngine(sc, precision=1)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True, tick_block=block)
+    it = b.interactions()
+    assert ((it["active"] == 1) & (it["master"] >= n)).sum() == n
+    for steps in (1, 11):
+        a.run(steps)
+        b.run(steps)
+        _same_run(a, b)
+    a.close()
+    b.close()

@@ -1452,7 +1452,17 @@ __device__ __forceinline__ void pairs_taken(const TickArgs& a) {
     const uint32_t nw = min(a.nwork[0], a.pcap), nww = min(a.nwork[-1], a.pcap - nw), count = KIND == 1 ? nw : nww;
     const uint32_t threads = gridDim.x * blockDim.x;
     auto item = [&](uint32_t q) { pair_item<LAW, XS, KIND>(a, a.pwork[KIND == 1 ? q : a.pcap - 1u - q]); };
-    if (count <= threads || (KIND == 1 && count <= 2u * threads && nww < count / 16u)) {
+    if (KIND == 2 && count <= threads) {
+        // a short list of wall pairs, a warp to every block in turn and not the first blocks full: FP64
+        // work, which holds up the SMs that those blocks share, the more the fewer SMs the launch found
+        // free (us a step from one engine to the next, the first blocks full and like this: hoppers of
+        // 60,000 spheres 50 to 52 and 44 to 46, of 100,000 71 to 79 and 58 to 64 at 64 threads a block,
+        // 69 to 71 and 54 to 57 at 256; 40,000-sphere drum 40 and 35)
+        const uint32_t q = (((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (threadIdx.x & 31u);
+        if (q < count) item(q);
+        return;
+    }
+    if (KIND == 1 && (count <= threads || (count <= 2u * threads && nww < count / 16u))) {
         for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += threads) item(q);
         return;
     }
