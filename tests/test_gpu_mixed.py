@@ -504,3 +504,18 @@ def test_wall_pairs_spread_over_the_blocks_and_in_chunks(n, block, engine_lib):
         _same_run(a, b)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,block", [(38911, 64), (38913, 64), (42000, 32), (48000, 64), (48000, 256)])
+def test_deferred_spheres_about_one_round_of_the_grid(n, block, engine_lib):
+    """Packings whose spheres, all deferred, just fit the split tick's grid with two threads each, and just
+    do not (one thread each then): against the pair pass, identical bits."""
+    sc = scenes.dense_pack(n=n, steps=1000)
+    a = engine_lib.GpuEngine(sc, precision=1, split_tick=True, tick_block=block)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True)
+    for k in (1, 11):
+        a.run(k)
+        b.run(k)
+        _same_run(a, b)
+    a.close()
+    b.close()

@@ -1143,23 +1143,33 @@ __global__ void __launch_bounds__(TPB) k_tick_each(TickArgs a) {
 
 // Threads per sphere of the full tick, as a power of two: 8 or 4 while that keeps every sphere resident
 // at once (`room` threads), 2 to five eighths of that many spheres, then 1 (launch_tick has the times).
-__host__ __device__ __forceinline__ int tick_lanes(uint64_t spheres, uint64_t room) {
+inline int tick_lanes(uint64_t spheres, uint64_t room) {
     int lanes = 8u * spheres <= 5u * room ? 1 : 0;
     while (lanes >= 1 && lanes < 3 && (spheres << (lanes + 1)) <= room) ++lanes;
     return lanes;
 }
 
+// ... of a deferred sphere: as many as keep all of them in one round of the grid.  The full tick goes on
+// with 2 a little past that (to five eighths of the spheres, where half would fit), as its blocks follow
+// one another; a grid of resident blocks that strides leaves most of them idle in its second round (us a
+// step by 2 and by 1 at 64 threads a block: 42,000 packed spheres 110 and 87, 48,000 115 and 86; 45,000
+// in a box 46 and 40).
+__device__ __forceinline__ int work_lanes(uint64_t spheres, uint64_t room) {
+    int lanes = 0;
+    while (lanes < 3 && (spheres << (lanes + 1)) <= room) ++lanes;
+    return lanes;
+}
+
 // The full tick of the split tick: a grid of the resident size takes the spheres the light kernel
-// deferred (none in a held step), spread over its threads as the full tick spreads a scene of that many.
-// (With one thread to a deferred sphere a 30,000-sphere hopper's step was 88 us, 2,000 packed spheres'
-// 95; 55 and 40 like this.)
+// deferred (none in a held step), spread over its threads.  (With one thread to a deferred sphere a
+// 30,000-sphere hopper's step was 88 us, 2,000 packed spheres' 95; 55 and 40 like this.)
 template <int LAW, bool XS>
 __global__ void __launch_bounds__(TPB, 2) k_tick_work(TickArgs a) {
     step_order();
     float2 vmax_local = make_float2(0.0f, 0.0f);
     if (!held_step(a)) {
         const uint32_t nw = *a.nwork;
-        const int lanes = tick_lanes(nw, (uint64_t)gridDim.x * blockDim.x);
+        const int lanes = work_lanes(nw, (uint64_t)gridDim.x * blockDim.x);
         const uint32_t B = blockDim.x >> lanes;
         for (uint32_t base = blockIdx.x * B; base < nw; base += gridDim.x * B) {
             vmax_local = fmax2(vmax_local, tick_block<LAW, XS>(a, lanes, base, min(B, nw - base), a.work));
