@@ -519,3 +519,20 @@ def test_deferred_spheres_about_one_round_of_the_grid(n, block, engine_lib):
         _same_run(a, b)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,block", [(77824, 64), (77825, 64), (100000, 128), (116736, 256), (116737, 256), (130000, 96)])
+def test_tick_of_dense_packings_about_the_resident_spheres(n, block, engine_lib):
+    """The full tick on both sides of the line past which a dense packing takes a thread per sphere, by
+    block size, against the pair pass: identical bits."""
+    sc = scenes.dense_pack(n=n, steps=1000)
+    a = engine_lib.GpuEngine(sc, precision=1, tick_block=block)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True)
+    for k in (1, 11):
+        a.run(k)
+        b.run(k)
+        sa, sb = a.state(), b.state()
+        for f in ("position", "velocity", "angular_velocity", "impact", "angular_impact"):
+            assert np.array_equal(sa[f], sb[f]), f
+    a.close()
+    b.close()

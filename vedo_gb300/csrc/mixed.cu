@@ -4006,12 +4006,14 @@ cudaError_t MixedEngine::launch_work(bool dep, void (*k)(TickArgs), void (*each)
 // loose spheres 12 / 12 / 12 / 14; 20,000 packed 71 / 55 / 64 / 69; 40,000-sphere drum 39 / 34 / 36 / 44;
 // 60,000 in the box 32 / 37, loose 13 / 15, packed 74 / 88, in a hopper 63 / 58; 200,000 packed 218 / 257.
 // A scene that leaves SMs without a block takes smaller blocks than tick_block, down to 64 threads
-// (2,000-sphere hopper, 256 to 64: 35 to 27).  From 2.5 times the resident spheres on, lists of ten
-// entries a sphere and more take the kernel with a thread per sphere (packings of 100,000 / 300,000: 121
-// against its 136, 284 against its 256).
+// (2,000-sphere hopper, 256 to 64: 35 to 27).  Lists of ten entries a sphere and more take the kernel with
+// a thread per sphere from one and a half times the resident spheres on, with blocks of up to 64 threads
+// from the resident spheres on (packings, us at 64 / 128 / 256 threads a block, spread and a thread each:
+// 78,000 117 / 114 / 114 and 110 / 109 / 112; 100,000 131 / 128 / 128 and 132 / 132 / 136; 125,000 151 /
+// 146 / 146 and 139 / 139 / 146; 180,000 214 / 208 / 208 and 180 / 180 / 191; 300,000 by 256 284 and 256).
 cudaError_t MixedEngine::launch_tick(bool dep, void (*k)(TickArgs, int), void (*each)(TickArgs), const TickArgs& a) {
     const uint64_t room = (uint64_t)sms_ * 512u;
-    if (2ull * n_ > 5u * room && nl_[nlc_].ne >= 10ull * n_)
+    if (2ull * n_ > (tpb_ <= 64 ? 2u : 3u) * room && nl_[nlc_].ne >= 10ull * n_)
         return step_launch(dep, each, (unsigned)((n_ + tpb_ - 1) / tpb_), (unsigned)tpb_, stream_, a);
     const int lanes = tick_lanes(n_, room);
     unsigned block = (unsigned)tpb_;
