@@ -165,3 +165,16 @@ def test_contact_activity_far_from_the_origin(away, periodic, engine_lib):
             assert len(set(first[pair].tolist())) == len(truth)
             assert e.observables()[9] == truth.sum()
         e.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [1, 255, 257, 8192, 8193, 155649])
+def test_observables_at_the_reductions_sizes(n, precision, engine_lib, port_lib):
+    """One partial sum, 2, 32, 33 and as many as there are blocks at most, a thread
+    over one object and more: the energies, extreme speeds and dispersions against the oracle's serial
+    sums, to their rounding (n half-ulps)."""
+    from oracle import PortWorld
+    sc = scenes.cluster(n=n, seed=n, walls="none", polydisperse=True)
+    e = engine_lib.GpuEngine(sc, precision=precision)
+    np.testing.assert_allclose(e.observables()[:9], PortWorld(sc).energy(), rtol=1e-13 + 1.2e-16 * n, atol=1e-40)
+    e.close()
