@@ -536,3 +536,21 @@ def test_tick_of_dense_packings_about_the_resident_spheres(n, block, engine_lib)
             assert np.array_equal(sa[f], sb[f]), f
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [1, 256, 257])
+def test_state_arrays_read_alone_and_together(n, precision, engine_lib):
+    """Any choice of state arrays, in any order, holds what a read of all of them holds."""
+    sc = scenes.cluster(n=n, seed=n, steps=1000)
+    e = engine_lib.GpuEngine(sc, precision=precision)
+    e.run(7)
+    whole = e.state()
+    fields = tuple(whole)
+    assert len(fields) == 7
+    for some in [(f,) for f in fields] + [fields[::-2], fields[5:], fields[1:4]]:
+        part = e.state(some)
+        assert tuple(part) == some
+        for f in some:
+            np.testing.assert_array_equal(part[f], whole[f])
+    e.close()

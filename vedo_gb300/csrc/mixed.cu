@@ -2617,7 +2617,7 @@ struct Fields {
     double* dst[7];
 };
 __global__ void __launch_bounds__(TPB) k_unpack3m(uint32_t n, uint32_t off, const uint32_t* __restrict__ int_of,
-                                                  Fields f) {
+                                                  const __grid_constant__ Fields f) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const double4_32a v = f.src[blockIdx.y][int_of[off + i]];
