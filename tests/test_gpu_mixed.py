@@ -554,3 +554,19 @@ def test_state_arrays_read_alone_and_together(n, precision, engine_lib):
         for f in some:
             np.testing.assert_array_equal(part[f], whole[f])
     e.close()
+
+
+@pytest.mark.parametrize("n,block", [(300, 96), (9000, 160), (19000, 224), (30000, 192), (45000, 96)])
+def test_spread_ticks_in_blocks_of_no_power_of_two(n, block, engine_lib):
+    """tick_block 96, 160, 192 and 224 with eight to one thread a sphere, the full and the split tick, against
+    the pair pass: identical bits."""
+    sc = scenes.hopper(n=n, seed=2, steps=1000, touching=True)
+    b = engine_lib.GpuEngine(sc, precision=1, pair_pass=True)
+    e = [engine_lib.GpuEngine(sc, precision=1, tick_block=block, split_tick=split) for split in (False, True)]
+    for k in (1, 11):
+        b.run(k)
+        for a in e:
+            a.run(k)
+            _same_run(a, b)
+    for x in e + [b]:
+        x.close()

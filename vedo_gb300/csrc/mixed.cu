@@ -4006,17 +4006,23 @@ cudaError_t MixedEngine::launch_work(bool dep, void (*k)(TickArgs), void (*each)
 // loose spheres 12 / 12 / 12 / 14; 20,000 packed 71 / 55 / 64 / 69; 40,000-sphere drum 39 / 34 / 36 / 44;
 // 60,000 in the box 32 / 37, loose 13 / 15, packed 74 / 88, in a hopper 63 / 58; 200,000 packed 218 / 257.
 // A scene that leaves SMs without a block takes smaller blocks than tick_block, down to 64 threads
-// (2,000-sphere hopper, 256 to 64: 35 to 27).  Lists of ten entries a sphere and more take the kernel with
-// a thread per sphere from one and a half times the resident spheres on, with blocks of up to 64 threads
-// from the resident spheres on (packings, us at 64 / 128 / 256 threads a block, spread and a thread each:
-// 78,000 117 / 114 / 114 and 110 / 109 / 112; 100,000 131 / 128 / 128 and 132 / 132 / 136; 125,000 151 /
-// 146 / 146 and 139 / 139 / 146; 180,000 214 / 208 / 208 and 180 / 180 / 191; 300,000 by 256 284 and 256).
+// (2,000-sphere hopper, 256 to 64: 35 to 27), and 192 counts as 128: two blocks of 192 leave a quarter of an
+// SM's registers empty, so a few blocks ran a second round (30,000-sphere box 36, 23 by 128; 30,000 packed
+// 78 and 55; the other sizes leave an eighth at most).  Lists of ten entries a sphere and more take the
+// kernel with a thread per sphere from one and a half times the resident spheres on, with blocks of up to
+// 64 threads from the resident spheres on (packings, us at 64 / 128 / 256 threads a block, spread and a
+// thread each: 78,000 117 / 114 / 114 and 110 / 109 / 112; 100,000 131 / 128 / 128 and 132 / 132 / 136;
+// 125,000 151 / 146 / 146 and 139 / 139 / 146; 180,000 214 / 208 / 208 and 180 / 180 / 191; 300,000 by 256
+// 284 and 256).  Shorter lists stay spread at every size: one wall contact a warp, or pairs unevenly
+// spread, cost a thread per sphere more (settled boxes of 43,000 / 64,000 / 216,000 48 / 46 / 127 spread and
+// 69 / 75 / 143 a thread each; hoppers 49 / 67 / 117 and 81 / 90 / 134) than the spreading costs a scene with
+// neither (the same boxes as an even lattice before their first wall contact 36 / 33 / 98 and 28 / 30 / 86).
 cudaError_t MixedEngine::launch_tick(bool dep, void (*k)(TickArgs, int), void (*each)(TickArgs), const TickArgs& a) {
     const uint64_t room = (uint64_t)sms_ * 512u;
     if (2ull * n_ > (tpb_ <= 64 ? 2u : 3u) * room && nl_[nlc_].ne >= 10ull * n_)
         return step_launch(dep, each, (unsigned)((n_ + tpb_ - 1) / tpb_), (unsigned)tpb_, stream_, a);
     const int lanes = tick_lanes(n_, room);
-    unsigned block = (unsigned)tpb_;
+    unsigned block = tpb_ == 192 ? 128u : (unsigned)tpb_;
     while (block >= 128u && block % 64u == 0u &&
            (((uint64_t)n_ << lanes) < (uint64_t)sms_ * block || (lanes == 0 && block > 128u)))
         block /= 2u;
