@@ -130,12 +130,19 @@ typedef struct vedo_scene_desc {
 } vedo_scene_desc;
 
 /* ---- engine options ---------------------------------------------------- */
-/* FP64: the drop-in; every FP64 operation in the reference's order, results bit-identical
- *       to the reference for the linear laws (Hertz-family laws and orbital walls within the
- *       last-ulp differences of pow, sin and cos).
+/* FP64: the drop-in; every FP64 operation that moves an object in the reference's order, results
+ *       bit-identical to the reference for the linear laws (Hertz-family laws and orbital walls
+ *       within the last-ulp differences of pow, sin and cos).  The spheres' orientations, which
+ *       nothing else reads, are the exception: they turn by the half-angle's Taylor terms, within
+ *       last bits of the reference's and nearer to the exact turn (4.3e-17 rms a step against
+ *       1.0e-16, at most 2.3e-15 after 1000 steps against 9e-14).
  * MIXED: contact forces in FP32 in pair-local coordinates, FP64 positions, velocities and
  *       overlap numerators, FP32 compensated sums per object; contact sets identical to
- *       FP64 at identical positions; sphere orientations are not integrated. */
+ *       FP64 at identical positions; sphere orientations are not integrated unless asked.
+ *       What vedo_gpu_get_interactions and the observables report is FP64's decision
+ *       everywhere.  The step's own is while coordinates stay within 1e5 radius sums of the
+ *       origin; farther out it can take a pair whose surfaces are up to 4e-15 of the
+ *       coordinate apart for touching, or one that overlaps by as little for apart. */
 enum { VEDO_PRECISION_FP64 = 0, VEDO_PRECISION_MIXED = 1 };
 
 typedef struct vedo_engine_opts {
@@ -157,8 +164,13 @@ typedef struct vedo_engine_opts {
                                  travel together may have used that up                  */
     uint32_t check_interval;  /* MIXED only: steps between displacement checks (10)   */
     uint32_t tick_block;      /* MIXED only: threads per block of the tick kernel, 32..256,
-                                 a multiple of 32 (0 = 256); a scene too small to give every
-                                 SM a block takes smaller ones                          */
+                                 a multiple of 32 (0 = 256).  The most a block holds, not
+                                 always its size: a scene too small to give every SM a block
+                                 takes smaller ones, the full tick takes 192 as 128, and where it
+                                 has one thread a list (above 5/8 of the threads resident at
+                                 once, 48,640 spheres on GB300) as well as in the split tick 192
+                                 and 256 run as 128 at most, except dense packings with a thread
+                                 per sphere                                              */
     float cell_scale;         /* MIXED only: cell edge as a multiple of 2 r_max + skin,
                                  >= 1 (0 = 1)                                          */
     uint32_t autotune;        /* MIXED only: 1 = the first steps of the run choose the tick
@@ -192,7 +204,7 @@ typedef struct vedo_engine_opts {
                                  turned by dt (w + dw/2) each step in FP64, as
                                  DOSphere::Response, DOSphere.cpp:40-44); 0 = leave them as
                                  they are (default: no force or contact depends on a sphere's
-                                 orientation, and the turn costs FP64 sines and cosines per
+                                 orientation, and the turn costs about 100 FP64 operations per
                                  spinning sphere per step).  The FP64 form always turns them */
     uint32_t persistent;      /* MIXED only: 1 = a check interval of steps runs as ONE cooperative
                                  launch (every block resident at once) whose stages are separated

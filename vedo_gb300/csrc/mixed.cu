@@ -1256,9 +1256,9 @@ __global__ void __launch_bounds__(TPB, 6) k_tick_light(TickArgs a) {   // 6 bloc
 }
 
 // DOSphere::Response (DOSphere.cpp:40-44): the orientation turns by dw = dt (w + dav/2) with the
-// angular velocity w before the step and its increment dav, by Vector3d::rotate_around in FP64 for
-// both axes; a zero turn leaves them.  Run after the tick when the caller asks for orientations,
-// from the new angular velocity w + dav and the increment: dt (w + dav - dav/2).
+// angular velocity w before the step and its increment dav, in FP64 for both axes, with the FP64 form's
+// operations (sphere_turn); a zero turn leaves them.  Run after the tick when the caller asks for
+// orientations, from the new angular velocity w + dav and the increment: dt (w + dav - dav/2).
 __device__ __forceinline__ void turn_sphere(const TickArgs& a, uint32_t i) {
     if (i >= a.n) return;
     const ModelDev& M = a.models[a.model_of[i]];
