@@ -1455,8 +1455,12 @@ __device__ __forceinline__ void pairs_from(const TickArgs& a, uint32_t first, ui
 // after the other, 320 like this; 1,000,000 packed spheres 508 to 480).  A list of at most a pair a thread is taken as it lies: every warp
 // asking at once costs about 1 ns each on the one counter (60,000-sphere hopper: 47 us a step so, 57
 // asking), and one of at most two where few wall pairs take room from it (60,000 spheres in a box: 32
-// against 40).  Longer ones go in about eight chunks a warp, the first of the blocks that surely start at
-// once fixed, the next one asked for before the present one is worked on.
+// against 40).  Longer ones go in about eight chunks a warp, of 64 pairs at most, the first of the blocks
+// that surely start at once fixed, the next one asked for before the present one is worked on.  (The list
+// follows the storage order, so the pairs at work at one time gather from one stretch of it: chunks of an
+// eighth of a warp's share spread that stretch past the L2.  us a step at 64 threads a block, eighths and 64
+// pairs: bed of 16,000,000 spheres in contact 4993 and 4696, 4,000,000 packed 1887 and 1694, 1,000,000 478
+// and 471; 256 hoppers by 256 1453 and 1408.)
 template <int LAW, bool XS, int KIND>
 __device__ __forceinline__ void pairs_taken(const TickArgs& a) {
     const uint32_t nw = min(a.nwork[0], a.pcap), nww = min(a.nwork[-1], a.pcap - nw), count = KIND == 1 ? nw : nww;
@@ -1477,7 +1481,7 @@ __device__ __forceinline__ void pairs_taken(const TickArgs& a) {
         return;
     }
     const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5, given = gridDim.x / 2u * wpb;
-    const uint32_t chunk = max(1u, count / (threads * 8u)) * 32u;
+    const uint32_t chunk = min(max(1u, count / (threads * 8u)), 2u) * 32u;
     uint32_t* const ctr = a.taken + (KIND == 1 ? 0 : 1);
     auto ask = [&]() { return lane == 0u ? given + atomicAdd(ctr, 1u) : 0u; };
     const uint32_t gw = blockIdx.x * wpb + (threadIdx.x >> 5);
